@@ -99,9 +99,8 @@ __global__ void __launch_bounds__(256) k_voxelize_na(GridView g, unsigned long l
     }
 }
 
-cudaError_t launch_tile_mask_view(const GridView& v, uint32_t* mask, int by, int bz, int tx, int ty, int tz,
-                                  cudaStream_t s);
-cudaError_t launch_trace_layout_view(const GridView& v, const TraceLayout& t, cudaStream_t s);
+cudaError_t launch_derive_view(const GridView& v, const TraceLayout& t, uint32_t* mask, int by, int bz, int tz,
+                               bool whole, cudaStream_t s);
 
 }  // namespace vxl
 
@@ -182,11 +181,8 @@ extern "C" vxl_status vxl_voxelize_noalloc(const vxl_grid_desc* gd, const vxl_mo
         VXL_TRY_CUDA(cudaGetLastError());
         i = j;
     }
-    VXL_TRY_CUDA(launch_tile_mask_view(v, gd->tile_mask, gd->by, gd->bz, gd->tx, gd->ty, gd->tz, s));
-    if (gd->trace_words) {
-        const TraceLayout t{gd->trace_words, gd->trace_lbx, gd->trace_lby, gd->trace_bz, gd->nx, gd->ny, gd->nz};
-        VXL_TRY_CUDA(launch_trace_layout_view(v, t, s));
-    }
+    const TraceLayout t{gd->trace_words, gd->trace_lbx, gd->trace_lby, gd->trace_bz, gd->nx, gd->ny, gd->nz};
+    VXL_TRY_CUDA(launch_derive_view(v, t, gd->tile_mask, gd->by, gd->bz, gd->tz, true, s));
     // the copies read the caller's host arrays: finish before returning them
     VXL_TRY_CUDA(cudaStreamSynchronize(s));
     return VXL_OK;
