@@ -10,10 +10,9 @@
 // this library holds until the process exits. Host code cannot use the array's
 // name as a device address, so the first call on each device looks the address
 // up with cudaGetSymbolAddress (with that device current) and keeps it.
-#include <climits>
 #include <mutex>
 
-#include "vxl_device.cuh"
+#include "voxel_tile.cuh"
 
 namespace vxl {
 
@@ -45,58 +44,22 @@ static vxl_status noalloc_tables(unsigned char** out) {
     return VXL_OK;
 }
 
-// Same mapping as k_voxelize (ShadowVoxSystem.cpp:137-177: fine voxel
-// ivec3((o + x*dx + y*dy + z*dz) * 10) for every model voxel with index >= 16,
-// SetVolumeAt bounds :83), launched without a chunk table:
-// blockIdx.y = instance first + y of a run with equal ops, blockIdx.x = chunk
-// of kVoxChunk source voxels (blocks past the model's last chunk return at once).
-__global__ void __launch_bounds__(256) k_voxelize_na(GridView g, unsigned long long* words,
-                                                     const DevInstance* __restrict__ inst,
-                                                     const DevModel* __restrict__ models, int first, int value,
-                                                     int32_t* aabb) {
+// The tiles of k_voxelize, launched without a table of them: blockIdx.y =
+// instance first + y of a run with equal ops, blockIdx.x = tile of its model
+// (blocks past the model's last tile return at once).
+__global__ void __launch_bounds__(kVoxThreads) k_voxelize_na(GridView g, unsigned long long* words,
+                                                             const DevInstance* __restrict__ inst,
+                                                             const DevModel* __restrict__ models, int first, int value,
+                                                             int32_t* aabb) {
+    __shared__ VoxTileShared sh;
     const int ii = first + (int)blockIdx.y;
     const DevInstance& I = inst[ii];
     const DevModel M = models[I.model];
-    const int sxy = M.sx * M.sy;
-    const int count = sxy * M.sz;
-    const int start = (int)blockIdx.x * kVoxChunk;
-    if (start >= count) return;  // uniform per block: no warp-level call below is skipped by part of a warp
-    const f3 o = mk(I.m[12], I.m[13], I.m[14]);
-    const f3 dx = mk(I.m[0] * 0.1f, I.m[1] * 0.1f, I.m[2] * 0.1f);
-    const f3 dy = mk(I.m[4] * 0.1f, I.m[5] * 0.1f, I.m[6] * 0.1f);
-    const f3 dz = mk(I.m[8] * 0.1f, I.m[9] * 0.1f, I.m[10] * 0.1f);
-    int mn[3] = {INT_MAX, INT_MAX, INT_MAX}, mx[3] = {INT_MIN, INT_MIN, INT_MIN};
-    for (int k = threadIdx.x; k < kVoxChunk; k += blockDim.x) {
-        const int v = start + k;
-        if (v >= count || M.data[v] < 16) continue;
-        const int z = v / sxy, r = v - z * sxy;
-        const int y = r / M.sx, x = r - y * M.sx;
-        const f3 wp = add(add(add(o, mul(dx, (float)x)), mul(dy, (float)y)), mul(dz, (float)z));
-        const int fx = (int)(wp.x * 10.0f), fy = (int)(wp.y * 10.0f), fz = (int)(wp.z * 10.0f);
-        mn[0] = min(mn[0], fx);
-        mn[1] = min(mn[1], fy);
-        mn[2] = min(mn[2], fz);
-        mx[0] = max(mx[0], fx);
-        mx[1] = max(mx[1], fy);
-        mx[2] = max(mx[2], fz);
-        if ((unsigned)fx < (unsigned)g.nx && (unsigned)fy < (unsigned)g.ny && (unsigned)fz < (unsigned)g.nz) {
-            const unsigned long long bit = 1ull << bit_index(fx, fy, fz);
-            if (value)
-                atomicOr(words + word_index(g, fx, fy, fz), bit);
-            else
-                atomicAnd(words + word_index(g, fx, fy, fz), ~bit);
-        }
-    }
-    if (aabb) {
-        for (int a = 0; a < 3; a++) {
-            const int lo = __reduce_min_sync(0xffffffffu, mn[a]);
-            const int hi = __reduce_max_sync(0xffffffffu, mx[a]);
-            if ((threadIdx.x & 31) == 0 && lo != INT_MAX) {
-                atomicMin(aabb + 6 * ii + a, lo);
-                atomicMax(aabb + 6 * ii + 3 + a, hi);
-            }
-        }
-    }
+    const VoxTileShape S = vox_tile_shape(M.sx);
+    auto up = [](int v, int l) { return ((uint32_t)v + (1u << l) - 1u) >> l; };
+    if ((uint64_t)blockIdx.x >= (uint64_t)up(M.sx, S.lx) * up(M.sy, S.ly) * up(M.sz, S.lz)) return;  // whole blocks
+    voxel_tile_init(sh);
+    voxel_tile(g, words, I.m, M, blockIdx.x, value != 0, aabb ? aabb + 6 * (size_t)ii : nullptr, sh);
 }
 
 cudaError_t launch_derive_view(const GridView& v, const TraceLayout& t, uint32_t* mask, int by, int bz, int tz,
@@ -169,14 +132,15 @@ extern "C" vxl_status vxl_voxelize_noalloc(const vxl_grid_desc* gd, const vxl_mo
     const DevModel* d_models = (const DevModel*)(tables + kNaInstBytes);
     // runs of equal ops, applied in array order (same result as one by one)
     for (int i = 0; i < n;) {
-        int j = i, maxchunks = 1;
+        int j = i;
+        uint64_t maxtiles = 1;
         while (j < n && instances[j].op == instances[i].op) {
             const vxl_model& m = models[instances[j].model];
-            long long c = ((long long)m.sx * m.sy * m.sz + kVoxChunk - 1) / kVoxChunk;
-            if (c > maxchunks) maxchunks = (int)c;
+            const uint64_t c = vox_tile_count(m.sx, m.sy, m.sz);
+            if (c > maxtiles) maxtiles = c;
             j++;
         }
-        k_voxelize_na<<<dim3((unsigned)maxchunks, (unsigned)(j - i)), 256, 0, s>>>(
+        k_voxelize_na<<<dim3((unsigned)maxtiles, (unsigned)(j - i)), kVoxThreads, 0, s>>>(
             v, (unsigned long long*)gd->words, d_inst, d_models, i, instances[i].op == VXL_OP_SET ? 1 : 0, d_aabb);
         VXL_TRY_CUDA(cudaGetLastError());
         i = j;

@@ -109,50 +109,141 @@ static vxl_status set_device(const vxl_ctx* ctx) {
 
 static bool grid_ok(const vxl_grid* g) { return g && g->ctx && g->words; }
 
-// Plan a voxelizer run: upload instances/models/chunk table, launch.
+// The cells an instance's image can touch, clipped to the grid: {least xyz,
+// greatest xyz}, empty when a least cell is above its greatest. The device's
+// mapping in the device's arithmetic (fp32, no contraction), every step of
+// which is monotone in the source coordinates, so two corners per axis bound
+// it; a placement that is not finite is taken to cover the grid.
+static void image_box(const float* m, const vxl_model& M, const vxl_grid* g, int* box) {
+    const int last[3] = {M.sx - 1, M.sy - 1, M.sz - 1}, n[3] = {g->nx, g->ny, g->nz};
+    for (int a = 0; a < 3; a++) {
+        const float d[3] = {m[a] * 0.1f, m[4 + a] * 0.1f, m[8 + a] * 0.1f};
+        for (int h = 0; h < 2; h++) {
+            float w = m[12 + a];
+            for (int k = 0; k < 3; k++) {
+                const float step = d[k] * (float)((d[k] >= 0.0f) == (h == 1) ? last[k] : 0);
+                w = w + step;
+            }
+            w = std::trunc(w * 10.0f);
+            box[3 * h + a] = w > -1.0f ? (w < (float)n[a] ? (int)w : n[a]) : -1;
+            if (!std::isfinite(w)) {
+                for (int k = 0; k < 3; k++) {
+                    box[k] = 0;
+                    box[3 + k] = n[k] - 1;
+                }
+                return;
+            }
+        }
+    }
+    for (int a = 0; a < 3; a++) {
+        box[a] = std::max(box[a], 0);
+        box[3 + a] = std::min(box[3 + a], n[a] - 1);
+    }
+}
+
+// Levels of instances: an instance comes after every earlier one of the other
+// op that may touch the same cells; all others commute with it. Moved
+// entities (a CLEAR and a SET each) take two levels unless they crowd, where
+// one launch per run of equal ops took two launches per entity. The pairwise
+// test is quadratic, so long mixed lists are ordered in segments of kSegment,
+// one after another. Returns the number of levels.
+static int voxel_levels(const vxl_grid* g, const vxl_model* models, const std::vector<DevInstance>& inst,
+                        std::vector<int>& level) {
+    const int n = (int)inst.size();
+    constexpr int kSegment = 1024;
+    level.assign((size_t)n, 0);
+    bool mixed = false;
+    for (int i = 1; i < n; i++) mixed |= inst[i].op != inst[0].op;
+    if (!mixed) return 1;
+    std::vector<int> boxes((size_t)6 * kSegment);
+    int top = 0;
+    for (int a = 0; a < n; a += kSegment) {
+        const int b = std::min(n, a + kSegment), base = top;
+        for (int i = a; i < b; i++) {
+            int* bi = &boxes[(size_t)6 * (i - a)];
+            image_box(inst[i].m, models[inst[i].model], g, bi);
+            int lv = base;
+            for (int j = a; j < i; j++) {
+                const int* bj = &boxes[(size_t)6 * (j - a)];
+                if (inst[j].op != inst[i].op && level[j] >= lv && std::max(bi[0], bj[0]) <= std::min(bi[3], bj[3]) &&
+                    std::max(bi[1], bj[1]) <= std::min(bi[4], bj[4]) && std::max(bi[2], bj[2]) <= std::min(bi[5], bj[5]))
+                    lv = level[j] + 1;
+            }
+            level[i] = lv;
+            top = std::max(top, lv + 1);
+        }
+    }
+    return top;
+}
+
+// Plan and launch a voxelizer call: one pinned image of its tables (jobs in
+// level order, tile counts before each, models, AABBs), one upload, one launch
+// per level. h_aabb (optional, host int32[n][6]) gives the AABBs' first values
+// and receives the results at the next synchronisation of the stream, in place
+// of d_aabb. Returns when the voxelization is done (the tables' host image and
+// the models are free again); the tile map and trace layout follow on the stream.
 static vxl_status voxelize_runs(vxl_ctx* ctx, vxl_grid* g, const vxl_model* models, int nmodels,
-                                const std::vector<DevInstance>& inst, int32_t* d_aabb, cudaStream_t s) {
+                                const std::vector<DevInstance>& inst, int32_t* d_aabb, cudaStream_t s,
+                                int32_t* h_aabb = nullptr) {
     const int n = (int)inst.size();
     if (n == 0) return VXL_OK;
-    std::vector<DevModel> dm((size_t)nmodels);
-    for (int i = 0; i < nmodels; i++) dm[i] = DevModel{models[i].data, models[i].sx, models[i].sy, models[i].sz, 0};
-    // chunk tables per run of equal ops, concatenated
-    std::vector<int2> chunks;
-    std::vector<std::pair<size_t, size_t>> runs;  // [begin, end) into chunks
-    std::vector<int> run_value;
-    for (int i = 0; i < n;) {
-        int j = i;
-        size_t b = chunks.size();
-        while (j < n && inst[j].op == inst[i].op) {
-            const DevModel& m = dm[inst[j].model];
-            long long cnt = (long long)m.sx * m.sy * m.sz;
-            for (long long v = 0; v < cnt; v += kVoxChunk) chunks.push_back(make_int2(j, (int)v));
-            j++;
-        }
-        runs.push_back({b, chunks.size()});
-        run_value.push_back(inst[i].op == VXL_OP_SET ? 1 : 0);
-        i = j;
-    }
-    size_t b_inst = inst.size() * sizeof(DevInstance);
-    size_t b_mod = dm.size() * sizeof(DevModel);
-    size_t b_ch = chunks.size() * sizeof(int2);
-    size_t off_mod = (b_inst + 255) & ~(size_t)255, off_ch = (off_mod + b_mod + 255) & ~(size_t)255;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    VXL_TRY_CUDA(cudaStreamIsCapturing(s, &cs));
+    if (cs != cudaStreamCaptureStatusNone) return fail(VXL_ERR_CUDA, "voxelize: not permitted while the stream is capturing");
+    std::vector<int> level;
+    const int nlev = voxel_levels(g, models, inst, level);
+    std::vector<int> at((size_t)nlev + 1, 0);  // jobs before each level
+    for (int i = 0; i < n; i++) at[(size_t)level[i] + 1]++;
+    for (int l = 0; l < nlev; l++) at[(size_t)l + 1] += at[l];
+    auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
+    const size_t o_first = al((size_t)n * sizeof(VoxJob)), o_mod = o_first + al(((size_t)n + 1) * sizeof(uint64_t));
+    const size_t o_box = o_mod + al((size_t)nmodels * sizeof(DevModel));
+    const size_t b_box = h_aabb ? (size_t)6 * n * sizeof(int32_t) : 0, total = o_box + b_box;
     void* scratch;
-    VXL_TRY(ctx_scratch(ctx, off_ch + b_ch + 256, &scratch));
-    char* base = (char*)scratch;
-    VXL_TRY_CUDA(cudaMemcpyAsync(base, inst.data(), b_inst, cudaMemcpyHostToDevice, s));
-    VXL_TRY_CUDA(cudaMemcpyAsync(base + off_mod, dm.data(), b_mod, cudaMemcpyHostToDevice, s));
-    if (b_ch) VXL_TRY_CUDA(cudaMemcpyAsync(base + off_ch, chunks.data(), b_ch, cudaMemcpyHostToDevice, s));
-    const DevInstance* d_inst = (const DevInstance*)base;
-    const DevModel* d_mod = (const DevModel*)(base + off_mod);
-    const int2* d_ch = (const int2*)(base + off_ch);
-    for (size_t r = 0; r < runs.size(); r++) {
-        int nch = (int)(runs[r].second - runs[r].first);
-        VXL_TRY(launch_voxelize_run(g, d_inst, d_mod, d_ch + runs[r].first, nch, run_value[r], d_aabb, s));
+    VXL_TRY(ctx_scratch(ctx, total, &scratch));
+    if (!ctx->vox_ev) VXL_TRY_CUDA(cudaEventCreateWithFlags(&ctx->vox_ev, cudaEventDisableTiming));
+    if (ctx->h_vox_bytes < total) {
+        if (ctx->h_vox) cudaFreeHost(ctx->h_vox);  // no call uses it any more: each waits for its own use
+        ctx->h_vox = nullptr;
+        ctx->h_vox_bytes = 0;
+        const size_t want = total + total / 2 + 4096;
+        VXL_TRY_CUDA(cudaHostAlloc(&ctx->h_vox, want, cudaHostAllocDefault));
+        ctx->h_vox_bytes = want;
     }
-    // the host vectors must outlive the async copies
-    VXL_TRY_CUDA(cudaStreamSynchronize(s));
-    return launch_build_tile_mask(g, s);
+    char* h = (char*)ctx->h_vox;
+    VoxJob* jobs = (VoxJob*)h;
+    uint64_t* first = (uint64_t*)(h + o_first);
+    DevModel* dm = (DevModel*)(h + o_mod);
+    std::vector<int> next(at.begin(), at.end() - 1);
+    for (int i = 0; i < n; i++) {
+        VoxJob& J = jobs[next[level[i]]++];
+        std::memcpy(J.m, inst[i].m, sizeof J.m);
+        J.model = inst[i].model;
+        J.op = inst[i].op == VXL_OP_SET ? 1 : 0;
+        J.index = i;
+        J.pad = 0;
+    }
+    first[0] = 0;
+    for (int k = 0; k < n; k++) {
+        const vxl_model& M = models[jobs[k].model];
+        first[k + 1] = first[k] + vox_tile_count(M.sx, M.sy, M.sz);
+    }
+    for (int i = 0; i < nmodels; i++) dm[i] = DevModel{models[i].data, models[i].sx, models[i].sy, models[i].sz, 0};
+    if (h_aabb) std::memcpy(h + o_box, h_aabb, b_box);
+    char* base = (char*)scratch;
+    VXL_TRY_CUDA(cudaMemcpyAsync(base, h, total, cudaMemcpyHostToDevice, s));
+    if (h_aabb) d_aabb = (int32_t*)(base + o_box);
+    for (int l = 0; l < nlev; l++)
+        VXL_TRY(launch_voxelize_level(g, (const VoxJob*)base, (const uint64_t*)(base + o_first),
+                                      (const DevModel*)(base + o_mod), at[l], at[(size_t)l + 1],
+                                      first[at[(size_t)l + 1]] - first[at[l]], d_aabb, s));
+    if (h_aabb) VXL_TRY_CUDA(cudaMemcpyAsync(h + o_box, d_aabb, b_box, cudaMemcpyDeviceToHost, s));
+    VXL_TRY_CUDA(cudaEventRecord(ctx->vox_ev, s));
+    // the tile map and the trace layout are queued before the wait, so the GPU goes on with them meanwhile
+    VXL_TRY(launch_build_tile_mask(g, s));
+    VXL_TRY_CUDA(cudaEventSynchronize(ctx->vox_ev));
+    if (h_aabb) std::memcpy(h_aabb, h + o_box, b_box);
+    return VXL_OK;
 }
 
 static vxl_status check_models(const vxl_model* models, int nmodels) {
@@ -256,6 +347,8 @@ vxl_status vxl_ctx_destroy(vxl_ctx* ctx) {
         cudaEventSynchronize(ctx->pev);
         cudaEventDestroy(ctx->pev);
     }
+    if (ctx->h_vox) cudaFreeHost(ctx->h_vox);
+    if (ctx->vox_ev) cudaEventDestroy(ctx->vox_ev);
     if (ctx->d_plist) cudaFree(ctx->d_plist);
     if (ctx->h_ptotal) cudaFreeHost(ctx->h_ptotal);
     if (ctx->h_pin) cudaFreeHost(ctx->h_pin);
@@ -880,11 +973,7 @@ vxl_status vxl_shadowvox_update(vxl_ctx* ctx, vxl_grid* g, const vxl_model* mode
         a[2] = sz - 1;
         a[3] = a[4] = a[5] = 0;
     }
-    void* st;
-    VXL_TRY(ctx_stage(ctx, h_aabb.size() * sizeof(int32_t), &st));
-    VXL_TRY_CUDA(cudaMemcpyAsync(st, h_aabb.data(), h_aabb.size() * sizeof(int32_t), cudaMemcpyHostToDevice, s));
-    VXL_TRY(voxelize_runs(ctx, g, models, nmodels, inst, (int32_t*)st, s));
-    VXL_TRY_CUDA(cudaMemcpyAsync(h_aabb.data(), st, h_aabb.size() * sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+    VXL_TRY(voxelize_runs(ctx, g, models, nmodels, inst, nullptr, s, h_aabb.data()));
     VXL_TRY_CUDA(cudaStreamSynchronize(s));
     if (h_regions) {
         for (int e = 0; e < n; e++) {
@@ -913,11 +1002,7 @@ vxl_status vxl_vox_destroyed(vxl_ctx* ctx, vxl_grid* g, const vxl_model* model, 
     inst[0].model = 0;
     inst[0].op = VXL_OP_CLEAR;
     int32_t h_aabb[6] = {sx - 1, sy - 1, sz - 1, 0, 0, 0};
-    void* st;
-    VXL_TRY(ctx_stage(ctx, sizeof h_aabb, &st));
-    VXL_TRY_CUDA(cudaMemcpyAsync(st, h_aabb, sizeof h_aabb, cudaMemcpyHostToDevice, s));
-    VXL_TRY(voxelize_runs(ctx, g, model, 1, inst, (int32_t*)st, s));
-    VXL_TRY_CUDA(cudaMemcpyAsync(h_aabb, st, sizeof h_aabb, cudaMemcpyDeviceToHost, s));
+    VXL_TRY(voxelize_runs(ctx, g, model, 1, inst, nullptr, s, h_aabb));
     VXL_TRY_CUDA(cudaStreamSynchronize(s));
     if (h_region) region_from_aabb(h_aabb, sx, sy, sz, h_region);
     return VXL_OK;

@@ -46,6 +46,10 @@ struct vxl_ctx {
     // positions and sky-masked normals rebuilt from a depth G-buffer
     void* d_fd;
     size_t fd_bytes;
+    // voxelizer: pinned image of its tables, and the event after the last call's use of them
+    void* h_vox;
+    size_t h_vox_bytes;
+    cudaEvent_t vox_ev;
     // fused lights: count and list of (pixel, light) pairs in range
     void* d_lpairs;
     size_t lpairs_bytes;
@@ -206,10 +210,36 @@ vxl_status launch_light_point(vxl_ctx* ctx, const vxl_grid* g, const float* wpos
                               const float* noise, int64_t npix, const float lp[3], float range, int spot,
                               float* shadow, vxl_ray_record* rec, cudaStream_t s);
 
-// one pass of instances that all carry the same op (they commute)
-vxl_status launch_voxelize_run(vxl_grid* g, const DevInstance* d_inst, const DevModel* d_models,
-                               const int2* d_chunks, int nchunks, int value, int32_t* d_aabb, cudaStream_t s);
+// A voxelizer instance in launch order, with its place in the caller's array.
+struct VoxJob {
+    float m[16];
+    int32_t model;
+    int32_t op;
+    int32_t index;
+    int32_t pad;
+};
+// jobs [job0, job1), whose writes commute; d_first: per job the tiles before it
+// (one more entry than jobs), ntiles of them in this range
+vxl_status launch_voxelize_level(vxl_grid* g, const VoxJob* d_jobs, const uint64_t* d_first, const DevModel* d_models,
+                                 int job0, int job1, uint64_t ntiles, int32_t* d_aabb, cudaStream_t s);
 
-constexpr int kVoxChunk = 1024;  // source voxels per voxelizer block
+// The voxelizer's tiles: 2^lx x 2^ly x 2^lz source voxels, 1024 of them, as
+// near a cube as lets a warp read runs of x (its image then covers few
+// bricks); narrow models take narrow tiles, which would otherwise be half
+// empty.
+struct VoxTileShape {
+    int lx, ly, lz;
+};
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+inline VoxTileShape vox_tile_shape(int sx) {
+    return sx > 8 ? VoxTileShape{4, 3, 3} : (sx > 4 ? VoxTileShape{3, 4, 3} : VoxTileShape{2, 4, 4});
+}
+inline uint64_t vox_tile_count(int sx, int sy, int sz) {
+    const VoxTileShape S = vox_tile_shape(sx);
+    auto up = [](int v, int l) { return ((uint64_t)v + (1u << l) - 1u) >> l; };
+    return up(sx, S.lx) * up(sy, S.ly) * up(sz, S.lz);
+}
 
 }  // namespace vxl
