@@ -1,25 +1,47 @@
 // trace.cu — occlusion tracing kernels: raw ray batches (DDA / Sparse /
 // SuperSparse), the DDA-mode occlusion pass over a G-buffer, and the
 // reference light passes (ambient, reflection, point/spot).
+#include "march_pool.cuh"
 #include "vxl_device.cuh"
 
 namespace vxl {
 
 // ------------------------------------------------------------ ray batches
-template <int MODE>
 __global__ void __launch_bounds__(128) k_trace_rays(GridView g, const float* __restrict__ rays, int64_t n,
                                                     vxl_ray_record* __restrict__ rec) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const float* q = rays + 7 * i;
-        f3 o = mk(q[0], q[1], q[2]), d = mk(q[3], q[4], q[5]);
-        float maxt = q[6];
-        Hit h;
-        if (MODE == VXL_MODE_DDA)
-            h = dda(g, o, d, maxt);
-        else
-            h = march(g, o, d, maxt, MODE == VXL_MODE_SPARSE ? 0.5f : 2.5f);
-        store_record(rec + i, h);
+        store_record(rec + i, dda(g, mk(q[0], q[1], q[2]), mk(q[3], q[4], q[5]), q[6]));
     }
+}
+
+// The marchers: `tile` rays (a multiple of 32) per warp.
+__global__ void __launch_bounds__(32 * kMarchWarps, kMarchBlocks) k_march_rays(const __grid_constant__ GridView g,
+                                                                    const float* __restrict__ rays, int64_t n,
+                                                                    uint32_t super, int tile,
+                                                                    vxl_ray_record* __restrict__ rec) {
+    __shared__ MarchPool pools[kMarchWarps];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t at = ((int64_t)blockIdx.x * kMarchWarps + warp) * tile;
+    MarchPool& P = pools[warp];
+    auto done = [&](uint32_t id, bool hit, float t, bool fine, f3 last, int steps) {
+        store_record(rec + at + id, march_hit(hit, t, fine, last, steps));
+    };
+    int count = 0;
+    for (int k = lane; k < tile; k += 32) {
+        const int64_t i = at + k;
+        f3 o = mk(0.0f, 0.0f, 0.0f), d = o;
+        float dist = 0.0f;
+        if (i < n) {
+            const float* q = rays + 7 * i;
+            o = mk(q[0], q[1], q[2]);
+            d = mk(q[3], q[4], q[5]);
+            dist = q[6];
+            if (!ray_domain_ok(o, d)) store_record(rec + i, Hit{0, 0, 0, dist, 0, 0});
+        }
+        march_push<true>(g, P, count, i < n, o, d, dist, (uint32_t)k | super, done);
+    }
+    march_pool<true>(g, P, count, done);
 }
 
 // ------------------------------------------------------ DDA-mode occlusion
@@ -114,58 +136,103 @@ __global__ void __launch_bounds__(128) k_occlusion(GridView g, const float* __re
 }
 
 // -------------------------------------------------- reference light passes
-// LightAmbient.frag:148-173
-__global__ void k_light_ambient(GridView g, const float* __restrict__ wcp_in, const float* __restrict__ nrm,
-                                const float* __restrict__ depth, const float4* __restrict__ noise, int64_t npix,
-                                f3 sun, float* __restrict__ shadow, float* __restrict__ irr,
-                                vxl_ray_record* __restrict__ rec) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < npix;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        float4 nz = noise[i];
-        f3 normal = ld3(nrm + 3 * i);
-        f3 wcp = ld3(wcp_in + 3 * i);
-        f3 randomVec = mul(cosine_sample(nz.x, nz.y), 0.1f);
-        randomVec.z *= glsl_sign(nz.z - 0.5f);
-        f3 wd = normalize(mix(sun, randomVec, 0.5f));
-        wcp = add(wcp, mul(wd, nz.w * 1.0f));
-        wcp = add(wcp, mul(randomVec, 2.5f));
-        float bias = smoothstep(0.0f, 0.2f, depth[i]) * 50.0f + 1.5f;
-        f3 o = add(wcp, mul(normal, bias));
-        Hit h0 = march(g, o, wd, 128.0f, 0.5f);
-        shadow[i] = (h0.t != 128.0f) ? 0.0f : 1.0f;
-        f3 T, B;
-        tangent_frame(normal, &T, &B);
-        f3 dir = frame_dir(T, B, normal, cosine_sample(nz.x, nz.y));
-        Hit h1 = march(g, o, dir, 128.0f, 2.5f);
-        float dd = h1.t / 128.0f;
-        irr[i] = dd * dd * 0.05f;
-        if (rec) {
-            store_record(rec + 2 * i, h0);
-            store_record(rec + 2 * i + 1, h1);
+// LightAmbient.frag:148-173: two rays a pixel, `tile` pixels (a multiple of
+// 32, two rays each in the pool) per warp.
+template <bool REC>
+__global__ void __launch_bounds__(32 * kMarchWarps, kMarchBlocks)
+    k_light_ambient(const __grid_constant__ GridView g, const float* __restrict__ wcp_in, const float* __restrict__ nrm,
+                    const float* __restrict__ depth, const float4* __restrict__ noise, int64_t npix, f3 sun, int tile,
+                    float* __restrict__ shadow, float* __restrict__ irr, vxl_ray_record* __restrict__ rec) {
+    __shared__ MarchPool pools[kMarchWarps];
+    __shared__ float res[kMarchWarps][kMarchRays];  // t of ray 2 * pixel + {0: sun, 1: hemisphere}
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t at = ((int64_t)blockIdx.x * kMarchWarps + warp) * tile;
+    MarchPool& P = pools[warp];
+    float* rt = res[warp];
+    auto done = [&](uint32_t id, bool hit, float t, bool fine, f3 last, int steps) {
+        if (hit) rt[id] = t;
+        if (REC) store_record(rec + 2 * at + id, march_hit(hit, t, fine, last, steps));
+    };
+    int count = 0;
+    for (int k = lane; k < tile; k += 32) {
+        const int64_t i = at + k;
+        f3 o = mk(0.0f, 0.0f, 0.0f), wd = o, dir = o;
+        if (i < npix) {
+            float4 nz = noise[i];
+            f3 normal = ld3(nrm + 3 * i);
+            f3 wcp = ld3(wcp_in + 3 * i);
+            const f3 cosv = cosine_sample(nz.x, nz.y);
+            f3 randomVec = mul(cosv, 0.1f);
+            randomVec.z *= glsl_sign(nz.z - 0.5f);
+            wd = normalize(mix(sun, randomVec, 0.5f));
+            wcp = add(wcp, mul(wd, nz.w * 1.0f));
+            wcp = add(wcp, mul(randomVec, 2.5f));
+            float bias = smoothstep(0.0f, 0.2f, depth[i]) * 50.0f + 1.5f;
+            o = add(wcp, mul(normal, bias));
+            f3 T, B;
+            tangent_frame(normal, &T, &B);
+            dir = frame_dir(T, B, normal, cosv);
+            rt[2 * k] = rt[2 * k + 1] = 128.0f;
+            if (REC) {
+                if (!ray_domain_ok(o, wd)) store_record(rec + 2 * i, Hit{0, 0, 0, 128.0f, 0, 0});
+                if (!ray_domain_ok(o, dir)) store_record(rec + 2 * i + 1, Hit{0, 0, 0, 128.0f, 0, 0});
+            }
         }
+        march_push<REC>(g, P, count, i < npix, o, wd, 128.0f, 2u * k, done);
+        march_push<REC>(g, P, count, i < npix, o, dir, 128.0f, (2u * k + 1u) | kMarchSuper, done);
+    }
+    march_pool<REC>(g, P, count, done);
+    __syncwarp();
+    for (int k = lane; k < tile; k += 32) {
+        const int64_t i = at + k;
+        if (i >= npix) break;
+        shadow[i] = (rt[2 * k] != 128.0f) ? 0.0f : 1.0f;
+        float dd = rt[2 * k + 1] / 128.0f;
+        irr[i] = dd * dd * 0.05f;
     }
 }
 
-// LightReflection.frag:92-113
-__global__ void k_light_reflection(GridView g, const float* __restrict__ wcp_in, const float* __restrict__ nrm,
-                                   const float* __restrict__ view_r, const float* __restrict__ rough,
-                                   const float4* __restrict__ noise, int64_t npix, float* __restrict__ t_out,
-                                   vxl_ray_record* __restrict__ rec) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < npix;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        float4 nz = noise[i];
-        f3 normal = ld3(nrm + 3 * i);
-        f3 wd = normalize(ld3(view_r + 3 * i));
-        f3 wcp = ld3(wcp_in + 3 * i);
-        f3 randomVec = cosine_sample(nz.x, nz.y);
-        randomVec.z *= glsl_sign(nz.z - 0.5f);
-        wd = mix(wd, randomVec, rough[i] * 0.1f);
-        wcp = add(wcp, mul(normal, nz.w));
-        wd = mul(wd, 1.0f + nz.w * 0.5f);
-        Hit h = march(g, add(wcp, normal), wd, 256.0f, 0.5f);
-        t_out[i] = h.t;
-        if (rec) store_record(rec + i, h);
+// LightReflection.frag:92-113, `tile` pixels (a multiple of 32) per warp
+template <bool REC>
+__global__ void __launch_bounds__(32 * kMarchWarps, kMarchBlocks)
+    k_light_reflection(const __grid_constant__ GridView g, const float* __restrict__ wcp_in,
+                       const float* __restrict__ nrm, const float* __restrict__ view_r,
+                       const float* __restrict__ rough, const float4* __restrict__ noise, int64_t npix, int tile,
+                       float* __restrict__ t_out, vxl_ray_record* __restrict__ rec) {
+    __shared__ MarchPool pools[kMarchWarps];
+    __shared__ float res[kMarchWarps][kMarchRays];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t at = ((int64_t)blockIdx.x * kMarchWarps + warp) * tile;
+    MarchPool& P = pools[warp];
+    float* rt = res[warp];
+    auto done = [&](uint32_t id, bool hit, float t, bool fine, f3 last, int steps) {
+        if (hit) rt[id] = t;
+        if (REC) store_record(rec + at + id, march_hit(hit, t, fine, last, steps));
+    };
+    int count = 0;
+    for (int k = lane; k < tile; k += 32) {
+        const int64_t i = at + k;
+        f3 o = mk(0.0f, 0.0f, 0.0f), wd = o;
+        if (i < npix) {
+            float4 nz = noise[i];
+            f3 normal = ld3(nrm + 3 * i);
+            wd = normalize(ld3(view_r + 3 * i));
+            f3 wcp = ld3(wcp_in + 3 * i);
+            f3 randomVec = cosine_sample(nz.x, nz.y);
+            randomVec.z *= glsl_sign(nz.z - 0.5f);
+            wd = mix(wd, randomVec, rough[i] * 0.1f);
+            wcp = add(wcp, mul(normal, nz.w));
+            wd = mul(wd, 1.0f + nz.w * 0.5f);
+            o = add(wcp, normal);
+            rt[k] = 256.0f;
+            if (REC && !ray_domain_ok(o, wd)) store_record(rec + i, Hit{0, 0, 0, 256.0f, 0, 0});
+        }
+        march_push<REC>(g, P, count, i < npix, o, wd, 256.0f, (uint32_t)k, done);
     }
+    march_pool<REC>(g, P, count, done);
+    __syncwarp();
+    for (int k = lane; k < tile; k += 32)
+        if (at + k < npix) t_out[at + k] = rt[k];
 }
 
 // LightPoint.frag:234-267 (spot = 0), LightSpot.frag:83-117 (spot = 1)
@@ -223,17 +290,17 @@ struct LightTable {
 };
 
 // The shadow ray of one (pixel, light) pair in range, as vxl_light_point traces
-// it (LightPoint.frag:105-129, LightSpot.frag:93-117): true when unshadowed.
-__device__ __forceinline__ bool light_pair_lit(const GridView& g, f3 worldPos, f3 normal, float4 nz, const LightDev& Lt,
-                                               f3 lightDir, float lightDistance) {
+// it (LightPoint.frag:105-129, LightSpot.frag:93-117): origin, direction and
+// length; step 2.5 for a spot light, 0.5 for a point light.
+__device__ __forceinline__ void light_pair_ray(f3 worldPos, f3 normal, float4 nz, const LightDev& Lt, f3 lightDir,
+                                               float lightDistance, f3* o, f3* dir, float* hitDist) {
     f3 wd;
-    float hitDist;
     if (Lt.spot) {
         wd = mul(normalize(lightDir), 10.0f);
-        hitDist = lightDistance * 10.0f;
+        *hitDist = lightDistance * 10.0f;
     } else {
         wd = lightDir;
-        hitDist = lightDistance * 10.5f;
+        *hitDist = lightDistance * 10.5f;
     }
     f3 wcp = mul(worldPos, 10.0f);
     f3 randomVec = mul(cosine_sample(nz.x, nz.y), 0.1f);
@@ -241,7 +308,16 @@ __device__ __forceinline__ bool light_pair_lit(const GridView& g, f3 worldPos, f
     wd = normalize(mix(wd, randomVec, 0.5f));
     wcp = add(wcp, mul(wd, nz.w * 1.0f));
     wcp = add(wcp, mul(randomVec, 2.5f));
-    const Hit h = march(g, add(wcp, mul(normal, 0.5f)), wd, hitDist, Lt.spot ? 2.5f : 0.5f);
+    *o = add(wcp, mul(normal, 0.5f));
+    *dir = wd;
+}
+// true when the pair is unshadowed
+__device__ __forceinline__ bool light_pair_lit(const GridView& g, f3 worldPos, f3 normal, float4 nz, const LightDev& Lt,
+                                               f3 lightDir, float lightDistance) {
+    f3 o, wd;
+    float hitDist;
+    light_pair_ray(worldPos, normal, nz, Lt, lightDir, lightDistance, &o, &wd, &hitDist);
+    const Hit h = march(g, o, wd, hitDist, Lt.spot ? 2.5f : 0.5f);
     return !(h.t < hitDist);
 }
 
@@ -354,25 +430,56 @@ __global__ void __launch_bounds__(256) k_light_points(GridView g, const float* _
     }
 }
 
-// Pass 2: the listed (pixel, light) pairs, one per thread.
-__global__ void __launch_bounds__(256) k_light_pairs(GridView g, const float* __restrict__ wpos,
-                                                     const float* __restrict__ nrm, const float4* __restrict__ noise,
-                                                     const __grid_constant__ LightTable T,
-                                                     const unsigned long long* __restrict__ pairs,
-                                                     const unsigned long long* __restrict__ npairs, uint64_t cap,
-                                                     unsigned long long* __restrict__ lit) {
+// Pass 2: the listed (pixel, light) pairs, up to kMarchRays per pool. The
+// list's length is known on the device only: few pairs are spread over all
+// warps of the launch in pools of 32 or 64.
+__global__ void __launch_bounds__(32 * kMarchWarps, kMarchBlocks)
+    k_light_pairs(const __grid_constant__ GridView g, const float* __restrict__ wpos, const float* __restrict__ nrm,
+                  const float4* __restrict__ noise, const __grid_constant__ LightTable T,
+                  const unsigned long long* __restrict__ pairs, const unsigned long long* __restrict__ npairs,
+                  uint64_t cap, unsigned long long* __restrict__ lit) {
+    __shared__ MarchPool pools[kMarchWarps];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    MarchPool& P = pools[warp];
     const unsigned long long n = *npairs < cap ? *npairs : cap;
-    for (unsigned long long e = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; e < n;
-         e += (unsigned long long)gridDim.x * blockDim.x) {
-        const unsigned long long pr = pairs[e];
-        const int64_t i = (int64_t)(pr >> 6);
-        const int l = (int)(pr & 63ull);
-        const LightDev& Lt = T.l[l];
-        const f3 worldPos = ld3(wpos + 3 * i);
-        const f3 lightDir = sub(Lt.pos, worldPos);
-        const float lightDistance = sqrtf(dot(lightDir, lightDir));
-        if (light_pair_lit(g, worldPos, ld3(nrm + 3 * i), noise[i], Lt, lightDir, lightDistance))
-            atomicOr(lit + i, 1ull << l);
+    const unsigned long long warps = (unsigned long long)gridDim.x * kMarchWarps;
+    int tile = kMarchRays;
+    while (tile > 32 && n < warps * tile) tile >>= 1;
+    for (unsigned long long at = ((unsigned long long)blockIdx.x * kMarchWarps + warp) * tile; at < n;
+         at += warps * tile) {
+        auto done = [&](uint32_t id, bool hit, float t, bool, f3, int) {
+            // a hit can lie at or beyond a short hitDist: the fine part always runs to 16
+            const unsigned long long pr = pairs[at + id];
+            const int64_t i = (int64_t)(pr >> 6);
+            const LightDev& Lt = T.l[(int)(pr & 63ull)];
+            if (hit) {
+                const f3 lightDir = sub(Lt.pos, ld3(wpos + 3 * i));
+                const float lightDistance = sqrtf(dot(lightDir, lightDir));
+                if (t < lightDistance * (Lt.spot ? 10.0f : 10.5f)) return;
+            }
+            atomicOr(lit + i, 1ull << (pr & 63ull));
+        };
+        int count = 0;
+        for (int k = lane; k < tile; k += 32) {
+            const bool on = at + k < n;
+            f3 o = mk(0.0f, 0.0f, 0.0f), wd = o;
+            float hitDist = 0.0f;
+            uint32_t id = (uint32_t)k;
+            if (on) {
+                const unsigned long long pr = pairs[at + k];
+                const int64_t i = (int64_t)(pr >> 6);
+                const LightDev& Lt = T.l[(int)(pr & 63ull)];
+                const f3 worldPos = ld3(wpos + 3 * i);
+                const f3 lightDir = sub(Lt.pos, worldPos);
+                light_pair_ray(worldPos, ld3(nrm + 3 * i), noise[i], Lt, lightDir, sqrtf(dot(lightDir, lightDir)), &o,
+                               &wd, &hitDist);
+                if (Lt.spot) id |= kMarchSuper;
+                // not marched (march_push): t = hitDist, unshadowed
+                if (!ray_domain_ok(o, wd) || march_gone(g, o, wd)) atomicOr(lit + i, 1ull << (pr & 63ull));
+            }
+            march_push<false>(g, P, count, on, o, wd, hitDist, id, done);
+        }
+        march_pool<false>(g, P, count, done);
     }
 }
 
@@ -385,17 +492,30 @@ static unsigned grid_blocks(vxl_ctx* ctx, int64_t n, int threads, int per_sm) {
     return (unsigned)need;
 }
 
+// Pixels (or rays) of a march kernel's warp: as many as its pool holds, fewer
+// (down to 32) while that would leave the GPU's warps without work: a pool's
+// lanes are busier the more rays it holds, but a call of few rays waits for
+// its slowest warp.
+static int march_tile(const vxl_ctx* ctx, int64_t n, int rays_each) {
+    int tile = kMarchRays / rays_each;
+    while (tile > 32 && n < (int64_t)ctx->sm_count * kMarchBlocks * kMarchWarps * tile) tile >>= 1;
+    return tile;
+}
+static unsigned march_blocks(int64_t n, int tile) {
+    return (unsigned)((n + (int64_t)tile * kMarchWarps - 1) / ((int64_t)tile * kMarchWarps));
+}
+
 vxl_status launch_trace_rays(vxl_ctx* ctx, const vxl_grid* g, const float* rays, int64_t n, int mode,
                              vxl_ray_record* rec, cudaStream_t s) {
     if (n <= 0) return VXL_OK;
     GridView v = view_of(g);
-    unsigned b = grid_blocks(ctx, n, 128, 16);
-    if (mode == VXL_MODE_DDA)
-        k_trace_rays<VXL_MODE_DDA><<<b, 128, 0, s>>>(v, rays, n, rec);
-    else if (mode == VXL_MODE_SPARSE)
-        k_trace_rays<VXL_MODE_SPARSE><<<b, 128, 0, s>>>(v, rays, n, rec);
-    else
-        k_trace_rays<VXL_MODE_SUPERSPARSE><<<b, 128, 0, s>>>(v, rays, n, rec);
+    if (mode == VXL_MODE_DDA) {
+        k_trace_rays<<<grid_blocks(ctx, n, 128, 16), 128, 0, s>>>(v, rays, n, rec);
+    } else {
+        const int tile = march_tile(ctx, n, 1);
+        k_march_rays<<<march_blocks(n, tile), 32 * kMarchWarps, 0, s>>>(v, rays, n, mode == VXL_MODE_SPARSE ? 0u : kMarchSuper,
+                                                                        tile, rec);
+    }
     ctx->launches++;
     VXL_TRY_CUDA(cudaGetLastError());
     return VXL_OK;
@@ -448,8 +568,9 @@ vxl_status launch_light_ambient(vxl_ctx* ctx, const vxl_grid* g, const float* wc
                                 vxl_ray_record* rec, cudaStream_t s) {
     if (npix <= 0) return VXL_OK;
     GridView v = view_of(g);
-    k_light_ambient<<<grid_blocks(ctx, npix, 128, 16), 128, 0, s>>>(v, wcp, nrm, depth, (const float4*)noise, npix,
-                                                                    sun_dir(), shadow, irr, rec);
+    const int tile = march_tile(ctx, npix, 2);
+    (rec ? k_light_ambient<true> : k_light_ambient<false>)<<<march_blocks(npix, tile), 32 * kMarchWarps, 0, s>>>(
+        v, wcp, nrm, depth, (const float4*)noise, npix, sun_dir(), tile, shadow, irr, rec);
     ctx->launches++;
     VXL_TRY_CUDA(cudaGetLastError());
     return VXL_OK;
@@ -460,8 +581,9 @@ vxl_status launch_light_reflection(vxl_ctx* ctx, const vxl_grid* g, const float*
                                    float* t, vxl_ray_record* rec, cudaStream_t s) {
     if (npix <= 0) return VXL_OK;
     GridView v = view_of(g);
-    k_light_reflection<<<grid_blocks(ctx, npix, 128, 16), 128, 0, s>>>(v, wcp, nrm, view_r, rough,
-                                                                       (const float4*)noise, npix, t, rec);
+    const int tile = march_tile(ctx, npix, 1);
+    (rec ? k_light_reflection<true> : k_light_reflection<false>)<<<march_blocks(npix, tile), 32 * kMarchWarps, 0, s>>>(
+        v, wcp, nrm, view_r, rough, (const float4*)noise, npix, tile, t, rec);
     ctx->launches++;
     VXL_TRY_CUDA(cudaGetLastError());
     return VXL_OK;
@@ -532,7 +654,7 @@ vxl_status launch_light_points(vxl_ctx* ctx, const vxl_grid* g, const float* wpo
     ctx->launches++;
     VXL_TRY_CUDA(cudaGetLastError());
     if (T.n > 0) {
-        k_light_pairs<<<(unsigned)ctx->sm_count * 8, 256, 0, s>>>(v, wpos, nrm, (const float4*)noise, T, pairs, npairs,
+        k_light_pairs<<<(unsigned)ctx->sm_count * kMarchBlocks, 32 * kMarchWarps, 0, s>>>(v, wpos, nrm, (const float4*)noise, T, pairs, npairs,
                                                                   cap, lit);
         ctx->launches++;
         VXL_TRY_CUDA(cudaGetLastError());
