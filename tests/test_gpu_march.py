@@ -1,4 +1,4 @@
-"""The pooled marchers (march_pool.cuh) against the oracle, bit for bit: pools of every fill, positions on the
+"""The pooled marchers (march_pool.cuh) and DDA rays against the oracle, bit for bit: pools of every fill, positions on the
 quarter-cell boundaries of the fetch, outside the grid and on its way out, lengths around the parts' limits."""
 import numpy as np
 import pytest
@@ -36,7 +36,7 @@ def _rays(dims, n, seed):
 
 # 700000 rays: the largest pools (below 622592 rays on this GPU they are smaller)
 @pytest.mark.parametrize("n", [1, 31, 33, 127, 129, 4097, 700000])
-@pytest.mark.parametrize("mode", [1, 2])
+@pytest.mark.parametrize("mode", [0, 1, 2])
 @pytest.mark.parametrize("dims", [(6, 10, 14), (130, 66, 34)])
 def test_ray_records(vxl, ctx, dims, mode, n):
     import torch
@@ -49,6 +49,24 @@ def test_ray_records(vxl, ctx, dims, mode, n):
     vxl.trace_rays(ctx, grid_from_r8(vxl, ctx, g), dev(rays), n, mode, rec)
     torch.cuda.synchronize()
     assert_recs_equal(recs_np(rec), oracle.trace_rays(g, rays, mode=mode), "mode %d" % mode)
+
+
+def test_dda_records_of_a_large_grid(vxl, ctx):
+    """Beyond 64 MiB of words the kernel keeps the current brick in registers."""
+    import torch
+
+    rng = np.random.default_rng(3)
+    g = np.zeros((65, 65, 16000), np.uint8)
+    for at in (slice(0, 40), slice(15960, 16000)):
+        g[:, :, at] = rng.choice(np.array([0, 0, 0, 0, 0, 1, 64, 130, 255], np.uint8), (65, 65, 40))
+    rays = _rays((130, 130, 130), 4097, 9)
+    rays[::2, 0] += np.float32(31870.0)
+    G = grid_from_r8(vxl, ctx, g)
+    assert G.describe().words_bytes > 64 << 20
+    rec = rec_buffer(len(rays))
+    vxl.trace_rays(ctx, G, dev(rays), len(rays), 0, rec)
+    torch.cuda.synchronize()
+    assert_recs_equal(recs_np(rec), oracle.trace_rays(g, rays, mode=0))
 
 
 @pytest.mark.parametrize("n", [1, 33, 5000, 640000])

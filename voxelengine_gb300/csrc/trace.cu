@@ -7,11 +7,105 @@
 namespace vxl {
 
 // ------------------------------------------------------------ ray batches
-__global__ void __launch_bounds__(128) k_trace_rays(GridView g, const float* __restrict__ rays, int64_t n,
-                                                    vxl_ray_record* __restrict__ rec) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const float* q = rays + 7 * i;
-        store_record(rec + i, dda(g, mk(q[0], q[1], q[2]), mk(q[3], q[4], q[5]), q[6]));
+// DDA rays with records. Independent rays end after very different step counts
+// (one ray a thread kept 19% of the lanes busy on rays from random points), so
+// a warp sets up 32 rays at a time in shared memory and its lanes take the next
+// one as theirs end; when the 32 are gone it sets up the next 32 beside the
+// rays still running. 1 M rays on a 384^3 grid: 415 -> 171 us (208 with pools
+// of 128 that each drain before the next). Issue-bound, 30 iterations a ray.
+constexpr int kRayBatch = 8;  // iterations between refills
+struct RayPool {
+    float4 a[32];  // cell (x, y as 16 bits each), t_max
+    float4 b[32];  // cell z and signs, t_delta
+    float maxt[32];
+    int lane[32];  // of the ray in its 32
+};
+
+template <bool CACHE>
+__global__ void __launch_bounds__(32 * kMarchWarps, kMarchBlocks)
+    k_trace_rays(const __grid_constant__ GridView g, const float* __restrict__ rays, int64_t n,
+                 vxl_ray_record* __restrict__ rec) {
+    __shared__ RayPool pools[kMarchWarps];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    RayPool& P = pools[warp];
+    int64_t next = ((int64_t)blockIdx.x * kMarchWarps + warp) * 32;  // first ray of the next 32
+    int64_t first = 0, id = 0;                                       // of the pool's 32; this lane's ray
+    int count = 0, base = 0;
+    DState s;
+    s.leap = false;
+    bool busy = false;
+    for (;;) {
+        const unsigned idle = __ballot_sync(0xffffffffu, !busy);
+        if (base == count && next < n) {
+            const int64_t i = next + lane;
+            bool on = i < n;
+            DState t;
+            if (on) {
+                const float* q = rays + 7 * i;
+                const f3 o = mk(q[0], q[1], q[2]), d = mk(q[3], q[4], q[5]);
+                if (ray_domain_ok(o, d) && dir_fast_ok(d)) {
+                    dda_init(t, o, d, q[6]);
+                    if ((unsigned)t.cx > g.ux || (unsigned)t.cy > g.uy || (unsigned)t.cz > g.uz) {
+                        // the first bounds test ends it
+                        store_record(rec + i, Hit{t.cx, t.cy, t.cz, 0.0f, 0, VXL_RF_EXIT_BOUNDS});
+                        on = false;
+                    }
+                } else {
+                    store_record(rec + i, dda(g, o, d, q[6]));  // a miss, or the literal form
+                    on = false;
+                }
+            }
+            const unsigned m = __ballot_sync(0xffffffffu, on);
+            if (on) {
+                const int at = __popc(m & march_lanes_below());
+                const int sg = (t.sx < 0 ? 1 : 0) | (t.sy < 0 ? 2 : 0) | (t.sz < 0 ? 4 : 0);
+                P.a[at] = make_float4(__int_as_float(t.cx | (t.cy << 16)), t.tx, t.ty, t.tz);
+                P.b[at] = make_float4(__int_as_float(t.cz | (sg << 16)), t.tdx, t.tdy, t.tdz);
+                P.maxt[at] = t.maxt;
+                P.lane[at] = lane;
+            }
+            first = next;
+            next += (int64_t)gridDim.x * kMarchWarps * 32;
+            base = 0;
+            count = __popc(m);
+            __syncwarp();
+        }
+        if (base < count) {
+            const int at = base + __popc(idle & march_lanes_below());
+            if (!busy && at < count) {
+                const float4 a = P.a[at], b = P.b[at];
+                const int xy = __float_as_int(a.x), zs = __float_as_int(b.x);
+                s.cx = xy & 0xffff;
+                s.cy = (int)((unsigned)xy >> 16);
+                s.cz = zs & 0xffff;
+                s.sx = (zs & 0x10000) ? -1 : 1;
+                s.sy = (zs & 0x20000) ? -1 : 1;
+                s.sz = (zs & 0x40000) ? -1 : 1;
+                s.tx = a.y;
+                s.ty = a.z;
+                s.tz = a.w;
+                s.tdx = b.y;
+                s.tdy = b.z;
+                s.tdz = b.w;
+                s.maxt = P.maxt[at];
+                s.tot = 0.0f;
+                s.n = 0;
+                s.wcur = 0xffffffffu;
+                id = first + P.lane[at];
+                busy = true;
+            }
+            base = min(base + __popc(idle), count);
+            __syncwarp();  // the slots are read before the next 32 rays are written
+        } else if (idle == 0xffffffffu && next >= n) {
+            break;
+        }
+        if (busy) {
+            Hit h;
+            if (dda_run<false, CACHE, !CACHE, true>(g, s, h, kRayBatch)) {
+                store_record(rec + id, h);
+                busy = false;
+            }
+        }
     }
 }
 
@@ -510,7 +604,9 @@ vxl_status launch_trace_rays(vxl_ctx* ctx, const vxl_grid* g, const float* rays,
     if (n <= 0) return VXL_OK;
     GridView v = view_of(g);
     if (mode == VXL_MODE_DDA) {
-        k_trace_rays<<<grid_blocks(ctx, n, 128, 16), 128, 0, s>>>(v, rays, n, rec);
+        // grids beyond 64 MiB of words keep the brick in registers, as the occlusion pool does
+        const unsigned b = (unsigned)std::min<int64_t>(march_blocks(n, 32), (int64_t)ctx->sm_count * kMarchBlocks);
+        (g->nwords > (8ull << 20) ? k_trace_rays<true> : k_trace_rays<false>)<<<b, 32 * kMarchWarps, 0, s>>>(v, rays, n, rec);
     } else {
         const int tile = march_tile(ctx, n, 1);
         k_march_rays<<<march_blocks(n, tile), 32 * kMarchWarps, 0, s>>>(v, rays, n, mode == VXL_MODE_SPARSE ? 0u : kMarchSuper,
