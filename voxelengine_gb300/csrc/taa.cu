@@ -5,14 +5,23 @@
 // engine's light images use its default linear filter) and sin/cos are the
 // library's own (sincos_own), as in the oracle.
 //
-// Every spiral tap samples six images at the same coordinates. A streaming
-// pre-pass (k_taa_pack) gathers the 16 floats a tap uses of each texel --
-// material, normal, depth, colour, motion and the light's rgb -- into four
-// float4 planes, so a bilinear tap is 16 vector loads instead of 40 loads
-// over six planar images; the interpolated values are the same floats
-// combined in the same order. Planes rather than 64-byte records: the 16-byte
-// loads of a warp's scattered taps then spread over eight L1 bank groups
-// (texel mod 8) instead of two.
+// Every spiral tap samples six images at the same coordinates, 16 floats of
+// four texels each. The L1 data pipe bounds the pass (a warp's taps land on
+// unrelated texels, so a 16-byte load costs about seven wavefronts), and what
+// helps is loading less, with the same floats combined in the same order:
+//  - a streaming pre-pass (k_taa_pack) packs (light rgb, depth), (colour,
+//    flags) and the normal as float4 planes, and notes per texel whether the
+//    four texels of a tap there have one colour, one normal and material: such
+//    a tap loads one texel's and interpolates that value with itself;
+//  - a tap whose colour differs from the pixel's has factor 0 (:119), so its
+//    normal and material are not loaded, unless a value near it is not finite
+//    (flagged too: 0 times that is not 0);
+//  - the motion test (> 0.1 apart, :120) needs no loads where the pre-pass's
+//    per-tile maxima show that no tap in reach can fail it.
+// 1080p: 1171 + 37 us (every tap 16 16-byte loads) -> 459 + 130 + 41 us, about
+// 60% issue-bound, the rest load latency.
+// Planes rather than records: the 16-byte loads of scattered taps then spread
+// over eight L1 bank groups (texel mod 8).
 #include "vxl_device.cuh"
 #include "vxl_internal.h"
 
@@ -78,29 +87,101 @@ __device__ __forceinline__ float dot3(const float* a, const float* b) {
     return d + a[2] * b[2];
 }
 
-// Texel planes (n texels each): q0 = material, q1 = (normal, depth),
-// q2 = (colour, motion.x), q3 = (light rgb, motion.y).
-constexpr int kTaaPlanes = 4;
+// Texel planes (n texels each): (light rgb, depth), (colour, flags), (normal, -).
+// The flags of texel (x, y) tell of the texels (x..x+1, y..y+1) inside the image.
+constexpr int kTaaPlanes = 3;
+constexpr int kTaaColor = 1;    // one colour, bit for bit
+constexpr int kTaaSurface = 2;  // one normal and one material
+constexpr int kTaaWild = 4;     // a value that is not below 1e15 in magnitude
+// bits 3-5, with kTaaSurface: the normal where it is a coordinate axis (2 * axis, + 1 for the negative one; 7: another)
+constexpr int kTaaNormal = 3, kTaaOther = 7;
+// bits 6-29, with kTaaSurface: the material in 1/63 steps, 6 bits a channel 
+constexpr int kTaaMaterial = 6, kTaaOdd = 1 << 30;  // kTaaOdd: no such material (not uniform, or outside [0, 1])
+constexpr int kPackW = 32, kPackH = 8;  // texels per block of the pre-pass
 
-__global__ void __launch_bounds__(256) k_taa_pack(const TaaIn I, float4* __restrict__ rec) {
-    const int n = I.W * I.H;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+__device__ __forceinline__ bool tame(float x) { return fabsf(x) < 1e15f; }
+
+// One texel a thread, with the row and column beyond the block's for the
+// flags. rec, per block the greatest |motion| component (a NaN counts as
+// infinite), and an empty list of disoccluded pixels. HBM-bound: 68 bytes read and 48 written per texel.
+__global__ void __launch_bounds__(kPackW* kPackH) k_taa_pack(const TaaIn I, float4* __restrict__ rec,
+                                                            float* __restrict__ motion_max, int* __restrict__ list) {
+    constexpr int SW = kPackW + 1, SH = kPackH + 1;
+    __shared__ float s_val[10][SW * SH];  // colour, normal, material
+    __shared__ bool s_wild[SW * SH];
+    __shared__ float s_max[kPackW * kPackH / 32];
+    const int t0 = threadIdx.x, x0 = blockIdx.x * kPackW, y0 = blockIdx.y * kPackH;
+    const size_t n = (size_t)I.W * I.H;
+    float top = 0.0f;
+    for (int t = t0; t < SW * SH; t += kPackW * kPackH) {
+        // texels of the block first, so that thread t0 holds texel t0 of the block
+        const bool own = t < kPackW * kPackH;
+        const int e = t - kPackW * kPackH;
+        const int lx = own ? t % kPackW : (e < SH ? kPackW : e - SH), ly = own ? t / kPackW : (e < SH ? e : kPackH);
+        const int x = min(x0 + lx, I.W - 1), y = min(y0 + ly, I.H - 1);
+        const size_t i = (size_t)y * I.W + x;
         const float4 m = __ldg(reinterpret_cast<const float4*>(I.material) + i);
         const float4 l = __ldg(reinterpret_cast<const float4*>(I.light) + i);
-        const float2 mo = __ldg(reinterpret_cast<const float2*>(I.motion) + i);
-        const float* nr = I.normal + 3 * (size_t)i;
-        const float* co = I.color + 3 * (size_t)i;
-        rec[i] = m;
-        rec[(size_t)n + i] = make_float4(__ldg(nr), __ldg(nr + 1), __ldg(nr + 2), __ldg(I.depth + i));
-        rec[2 * (size_t)n + i] = make_float4(__ldg(co), __ldg(co + 1), __ldg(co + 2), mo.x);
-        rec[3 * (size_t)n + i] = make_float4(l.x, l.y, l.z, mo.y);
+        const float v[10] = {__ldg(I.color + 3 * i),      __ldg(I.color + 3 * i + 1),  __ldg(I.color + 3 * i + 2),
+                             __ldg(I.normal + 3 * i),     __ldg(I.normal + 3 * i + 1), __ldg(I.normal + 3 * i + 2),
+                             m.x, m.y, m.z, m.w};
+        const float de = __ldg(I.depth + i);
+        bool ok = tame(l.x) && tame(l.y) && tame(l.z) && tame(de);
+#pragma unroll
+        for (int k = 0; k < 10; k++) {
+            ok = ok && tame(v[k]);
+            s_val[k][ly * SW + lx] = v[k];
+        }
+        s_wild[ly * SW + lx] = !ok;
+        if (own && x0 + lx < I.W && y0 + ly < I.H) {
+            rec[i] = make_float4(l.x, l.y, l.z, de);
+            rec[2 * n + i] = make_float4(v[3], v[4], v[5], 0.0f);
+            const float2 mo = __ldg(reinterpret_cast<const float2*>(I.motion) + i);
+            const float a = fabsf(mo.x), b = fabsf(mo.y);
+            top = a == a && b == b ? fmaxf(a, b) : INFINITY;
+        }
+    }
+    for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+    if ((t0 & 31) == 0) s_max[t0 >> 5] = top;
+    __syncthreads();
+    const int lx = t0 % kPackW, ly = t0 / kPackW, c = ly * SW + lx;
+    if (x0 + lx < I.W && y0 + ly < I.H) {
+        const int q[3] = {c + 1, c + SW, c + SW + 1};
+        bool color = true, surface = true, wild = s_wild[c];
+#pragma unroll
+        for (int j = 0; j < 3; j++) {
+#pragma unroll
+            for (int k = 0; k < 10; k++) {
+                const bool same = __float_as_uint(s_val[k][c]) == __float_as_uint(s_val[k][q[j]]);
+                if (k < 3) color = color && same;
+                else surface = surface && same;
+            }
+            wild = wild || s_wild[q[j]];
+        }
+        int axis = kTaaOther, bins = 0;
+        bool small = true;
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const float m = s_val[6 + k][c];
+            small = small && m >= 0.0f && m <= 1.0f;
+            bins |= (int)(m * 63.0f) << (6 * k);
+        }
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            const uint32_t v = __float_as_uint(s_val[3 + k][c]) & 0x7fffffffu;
+            const uint32_t rest = __float_as_uint(s_val[3 + (k + 1) % 3][c]) | __float_as_uint(s_val[3 + (k + 2) % 3][c]);
+            if (v == 0x3f800000u && rest == 0u) axis = 2 * k + (s_val[3 + k][c] < 0.0f ? 1 : 0);
+        }
+        const int f = (wild ? kTaaWild : 0) | (color ? kTaaColor : 0) |
+                      (surface ? kTaaSurface | (axis << kTaaNormal) | (small ? bins << kTaaMaterial : kTaaOdd) : kTaaOdd);
+        rec[n + (size_t)(y0 + ly) * I.W + x0 + lx] = make_float4(s_val[0][c], s_val[1][c], s_val[2][c], __int_as_float(f));
+    }
+    if (t0 == 0) {
+        if (blockIdx.x == 0 && blockIdx.y == 0) list[0] = 0;
+        for (int w = 1; w < kPackW * kPackH / 32; w++) top = fmaxf(top, s_max[w]);
+        motion_max[blockIdx.y * gridDim.x + blockIdx.x] = top;
     }
 }
-
-// One bilinear tap of every image a spiral / neighbourhood sample reads.
-struct Tap {
-    float mo[2], co[3], no[3], ma[4], de, li[3];
-};
 
 __device__ __forceinline__ void lerp4(const float4& a, const float4& b, const float4& c, const float4& d, float ax,
                                       float bx, float ay, float by, float* o) {
@@ -114,40 +195,46 @@ __device__ __forceinline__ void lerp4(const float4& a, const float4& b, const fl
     }
 }
 
-// The same coordinates, clamping and weights as tex4, over the planes.
-__device__ __forceinline__ void tap(const float4* __restrict__ rec, int W, int H, float u, float v, Tap* t) {
-    const float x = u * (float)W - 0.5f, y = v * (float)H - 0.5f;
-    const float fx = floorf(x), fy = floorf(y);
-    const float ax = x - fx, ay = y - fy;
-    int x0 = (int)fx, y0 = (int)fy, x1 = x0 + 1, y1 = y0 + 1;
-    x0 = x0 < 0 ? 0 : (x0 > W - 1 ? W - 1 : x0);
-    x1 = x1 < 0 ? 0 : (x1 > W - 1 ? W - 1 : x1);
-    y0 = y0 < 0 ? 0 : (y0 > H - 1 ? H - 1 : y0);
-    y1 = y1 < 0 ? 0 : (y1 > H - 1 ? H - 1 : y1);
-    const float bx = 1.0f - ax, by = 1.0f - ay;
-    const size_t n = (size_t)W * H;
-    const float4* r00 = rec + ((size_t)y0 * W + x0);
-    const float4* r10 = rec + ((size_t)y0 * W + x1);
-    const float4* r01 = rec + ((size_t)y1 * W + x0);
-    const float4* r11 = rec + ((size_t)y1 * W + x1);
-    float o[4];
-    lerp4(__ldg(r00), __ldg(r10), __ldg(r01), __ldg(r11), ax, bx, ay, by, t->ma);
-    lerp4(__ldg(r00 + n), __ldg(r10 + n), __ldg(r01 + n), __ldg(r11 + n), ax, bx, ay, by, o);
-    t->no[0] = o[0];
-    t->no[1] = o[1];
-    t->no[2] = o[2];
-    t->de = o[3];
-    lerp4(__ldg(r00 + 2 * n), __ldg(r10 + 2 * n), __ldg(r01 + 2 * n), __ldg(r11 + 2 * n), ax, bx, ay, by, o);
-    t->co[0] = o[0];
-    t->co[1] = o[1];
-    t->co[2] = o[2];
-    t->mo[0] = o[3];
-    lerp4(__ldg(r00 + 3 * n), __ldg(r10 + 3 * n), __ldg(r01 + 3 * n), __ldg(r11 + 3 * n), ax, bx, ay, by, o);
-    t->li[0] = o[0];
-    t->li[1] = o[1];
-    t->li[2] = o[2];
-    t->mo[1] = o[3];
-}
+// A tap's place: the coordinates, clamping and weights of tex4.
+struct TapAt {
+    int i00, dx, dy;  // texel (x0, y0), offsets to x1 and y1
+    float ax, ay, bx, by;
+    __device__ __forceinline__ TapAt(int W, int H, float u, float v) {
+        const float x = u * (float)W - 0.5f, y = v * (float)H - 0.5f;
+        const float fx = floorf(x), fy = floorf(y);
+        ax = x - fx;
+        ay = y - fy;
+        int x0 = (int)fx, y0 = (int)fy, x1 = x0 + 1, y1 = y0 + 1;
+        x0 = x0 < 0 ? 0 : (x0 > W - 1 ? W - 1 : x0);
+        x1 = x1 < 0 ? 0 : (x1 > W - 1 ? W - 1 : x1);
+        y0 = y0 < 0 ? 0 : (y0 > H - 1 ? H - 1 : y0);
+        y1 = y1 < 0 ? 0 : (y1 > H - 1 ? H - 1 : y1);
+        bx = 1.0f - ax;
+        by = 1.0f - ay;
+        i00 = y0 * W + x0;
+        dx = x1 - x0;
+        dy = (y1 - y0) * W;
+    }
+    // a float4 image here; a: its texel (x0, y0), which all four equal where `one`
+    __device__ __forceinline__ void get(const float4* __restrict__ img, float4 a, bool one, float* o) const {
+        float4 b = a, c = a, d = a;
+        if (!one) {
+            const float4* q = img + i00;
+            b = __ldg(q + dx);
+            c = __ldg(q + dy);
+            d = __ldg(q + dx + dy);
+        }
+        lerp4(a, b, c, d, ax, bx, ay, by, o);
+    }
+    __device__ __forceinline__ void motion(const float* __restrict__ img, float* o) const {
+        const float2* q = reinterpret_cast<const float2*>(img) + i00;
+        const float2 a = __ldg(q), b = __ldg(q + dx), c = __ldg(q + dy), d = __ldg(q + dx + dy);
+        const float tx = a.x * bx + b.x * ax, ux = c.x * bx + d.x * ax;
+        const float ty = a.y * bx + b.y * ax, uy = c.y * bx + d.y * ax;
+        o[0] = tx * by + ux * ay;
+        o[1] = ty * by + uy * ay;
+    }
+};
 
 // Centre values a disocclusion tap compares against.
 struct Centre {
@@ -156,57 +243,153 @@ struct Centre {
 
 // One tap (x, y) of the 19x19 disocclusion neighbourhood (LightTAA.frag:61-80):
 // (factor * light.rgb, factor), the terms its sums add in order.
-__device__ __forceinline__ float4 disocc_tap(const float4* __restrict__ rec, int W, int H, float iResx, float iResy,
-                                             const Centre& c, int x, int y) {
+__device__ __forceinline__ float4 disocc_tap(const TaaIn& I, const float4* __restrict__ rec, float iResx, float iResy,
+                                             const Centre& c, bool wild, int x, int y) {
     const float FAR = 4096.0f;
     const float ox = (float)x * iResx, oy = (float)y * iResy;
     const float u = clampg(c.uvx + ox, 0.001f, 0.999f), v = clampg(c.uvy + oy, 0.001f, 0.999f);
-    Tap t;
-    tap(rec, W, H, u, v, &t);
-    float factor = gmax(dot3(c.no, t.no), 0.0f);
-    factor *= glsl_step(0.8f, 1.0f - len4(c.ma, t.ma));
-    factor *= 1.0f - clampg(fabsf(c.de - t.de) * FAR, 0.0f, 1.0f);
-    factor *= 1.0f - clampg(len3(c.co, t.co), 0.0f, 1.0f);
-    if (len2(c.mo[0] - t.mo[0], c.mo[1] - t.mo[1]) > 0.1f) factor = 0.0f;
-    return make_float4(factor * t.li[0], factor * t.li[1], factor * t.li[2], factor);
+    const TapAt t(I.W, I.H, u, v);
+    const size_t n = (size_t)I.W * I.H;
+    const float4* mat = reinterpret_cast<const float4*>(I.material);
+    const float4 c00 = __ldg(rec + n + t.i00);
+    const int f = __float_as_int(c00.w);
+    float ld[4], co[4], no[4], ma[4], mo[2];
+    t.get(mat, __ldg(mat + t.i00), f & kTaaSurface, ma);
+    const float like = glsl_step(0.8f, 1.0f - len4(c.ma, ma));
+    if (like == 0.0f && !wild && !(f & kTaaWild)) return make_float4(0.0f, 0.0f, 0.0f, 0.0f);  // adds nothing
+    t.get(rec, __ldg(rec + t.i00), false, ld);
+    t.get(rec + n, c00, f & kTaaColor, co);
+    t.get(rec + 2 * n, __ldg(rec + 2 * n + t.i00), f & kTaaSurface, no);
+    t.motion(I.motion, mo);
+    float factor = gmax(dot3(c.no, no), 0.0f);
+    factor *= like;
+    factor *= 1.0f - clampg(fabsf(c.de - ld[3]) * FAR, 0.0f, 1.0f);
+    factor *= 1.0f - clampg(len3(c.co, co), 0.0f, 1.0f);
+    if (len2(c.mo[0] - mo[0], c.mo[1] - mo[1]) > 0.1f) factor = 0.0f;
+    return make_float4(factor * ld[0], factor * ld[1], factor * ld[2], factor);
 }
 
+// 1.212 - radius / 12 of the spiral's taps (LightTAA.frag:115)
+__constant__ float c_ring[12] = {1.212f - 2.0f / 12.0f, 1.212f - 3.0f / 12.0f,  1.212f - 4.0f / 12.0f,  1.212f - 5.0f / 12.0f,
+                                 1.212f - 6.0f / 12.0f, 1.212f - 7.0f / 12.0f,  1.212f - 8.0f / 12.0f,  1.212f - 9.0f / 12.0f,
+                                 1.212f - 10.0f / 12.0f, 1.212f - 11.0f / 12.0f, 1.212f - 12.0f / 12.0f, 1.212f - 13.0f / 12.0f};
+
 constexpr int kDisTaps = 19 * 19;
-constexpr int kDisCoopMax = 16;  // warps with more disoccluded pixels run them one per lane
+
+// The centre of a pixel: everything its taps are compared with; returns its flags.
+__device__ __forceinline__ int taa_centre(const TaaIn& I, const float4* __restrict__ rec, int px, int py, Centre& c) {
+    const size_t n = (size_t)I.W * I.H;
+    const float4* mat = reinterpret_cast<const float4*>(I.material);
+    c.uvx = ((float)px + 0.5f) / (float)I.W;
+    c.uvy = ((float)py + 0.5f) / (float)I.H;
+    const TapAt t(I.W, I.H, c.uvx, c.uvy);
+    float q[4];
+    const float4 c00 = __ldg(rec + n + t.i00);
+    const int f = __float_as_int(c00.w);
+    t.get(rec + n, c00, f & kTaaColor, q);
+    c.co[0] = q[0];
+    c.co[1] = q[1];
+    c.co[2] = q[2];
+    t.get(rec + 2 * n, __ldg(rec + 2 * n + t.i00), f & kTaaSurface, q);
+    c.no[0] = q[0];
+    c.no[1] = q[1];
+    c.no[2] = q[2];
+    t.get(mat, __ldg(mat + t.i00), f & kTaaSurface, c.ma);
+    t.get(rec, __ldg(rec + t.i00), false, q);
+    c.de = q[3];
+    t.motion(I.motion, c.mo);
+    return f;
+}
+
+// The pixels whose reprojection leaves the screen (listed by k_taa), up to
+// kEdgeGroup at a time per block: the current frame's 19x19 neighbourhood only.
+// The threads compute a pixel's taps row by row (their texels are then
+// adjacent) into shared memory, and four lanes per pixel add its four sums up
+// column by column, the shader's loop order, so the result is the same float.
+// 361 taps instead of 12: inside the spiral's kernel the few warps with such
+// pixels, at the screen's edge, ran on after all others (1080p, 1% of the
+// pixels: 958 us, now 459 for the spiral and 130 here).
+constexpr int kEdgeGroup = 4;
+__global__ void __launch_bounds__(128) k_taa_edge(const TaaIn I, const float4* __restrict__ rec,
+                                                  const int* __restrict__ list, float* __restrict__ out) {
+    __shared__ float4 s_dis[kEdgeGroup][kDisTaps];
+    __shared__ Centre s_centre[kEdgeGroup];
+    __shared__ int s_flags[kEdgeGroup];
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const float iResx = 1.0f / (float)I.W, iResy = 1.0f / (float)I.H;
+    const int count = list[0];
+    const int group = min(kEdgeGroup, (count + (int)gridDim.x - 1) / (int)gridDim.x);
+    for (int k = blockIdx.x * group; k < count; k += gridDim.x * group) {
+        const int m = min(group, count - k);
+        if (wib < m) {
+            const int i = list[1 + k + wib];
+            Centre c;
+            const int f = taa_centre(I, rec, i % I.W, i / I.W, c);
+            if (lane == 0) {
+                s_centre[wib] = c;
+                s_flags[wib] = f;
+            }
+        }
+        __syncthreads();
+        for (int e = 0; e < m; e++)
+            for (int t = threadIdx.x; t < kDisTaps; t += 128) {
+                const int x = t % 19, y = t / 19;
+                s_dis[e][x * 19 + y] = disocc_tap(I, rec, iResx, iResy, s_centre[e], s_flags[e] & kTaaWild, x - 9, y - 9);
+            }
+        __syncthreads();
+        if (wib == 0) {
+            float acc = 0.0f;
+            if (lane < 4 * m) {
+                const float* f = reinterpret_cast<const float*>(s_dis[lane >> 2]) + (lane & 3);
+                for (int x = 0; x < 19; x++) {
+#pragma unroll
+                    for (int y = 0; y < 19; y++) acc += f[4 * (x * 19 + y)];
+                }
+            }
+            const float total = __shfl_sync(0xffffffffu, acc, lane | 3);
+            if (lane < 4 * m)
+                out[4 * (size_t)list[1 + k + (lane >> 2)] + (lane & 3)] = (lane & 3) < 3 ? acc / total : 1.0f;
+        }
+        __syncthreads();
+    }
+}
+
+// Reach of a pixel's taps, in texels, within which the motion test is decided
+// by the pre-pass's maxima: they lie at most 14.5 away, their texels at most
+// 16, so the block's own and its neighbouring tiles of 32 x 8 hold them, two
+// rows of tiles up and down. Motions below 0.035 differ by less than 0.1.
+constexpr float kTaaReach = 14.5f, kTaaStill = 0.035f;
 
 // 32x4-pixel blocks: the spiral taps of neighbouring pixels overlap in L1.
-// A pixel whose reprojection leaves the screen samples 361 taps instead of 12;
-// when a warp holds few such pixels, all 32 lanes compute each one's taps
-// (x-major order, as the shader's loops) into shared memory and lanes 0-3
-// add the four sums up in that order, so the result is the same float.
-__global__ void __launch_bounds__(128) k_taa(const TaaIn I, const float4* __restrict__ rec, float* __restrict__ out) {
-    __shared__ float4 s_dis[4][kDisTaps];
+// Four rows and 7 blocks per SM (72 registers, 48 bytes of spills) measured
+// 459 us at 1080p; 6 blocks 504, 8 blocks 484, two rows 484, eight rows 510.
+constexpr int kTaaRows = 4;
+__global__ void __launch_bounds__(32 * kTaaRows, 7) k_taa(const TaaIn I, const float4* __restrict__ rec,
+                                             const float* __restrict__ motion_max, int* __restrict__ list,
+                                                         float* __restrict__ out) {
     const int W = I.W, H = I.H;
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    const int px = blockIdx.x * 32 + lane, py = blockIdx.y * 4 + wib;
+    const int px = blockIdx.x * 32 + lane, py = blockIdx.y * kTaaRows + wib;
     const bool valid = px < W && py < H;
     const int i = valid ? py * W + px : 0;
+    const size_t n = (size_t)W * H;
+    const float4* mat = reinterpret_cast<const float4*>(I.material);
+    bool still = W <= 14000 && H <= 14000;
+    if (lane < 15) {
+        const int tx = (int)blockIdx.x - 1 + lane % 3, ty = (int)(blockIdx.y * kTaaRows / kPackH) - 2 + lane / 3;
+        const int nx = (W + kPackW - 1) / kPackW, ny = (H + kPackH - 1) / kPackH;
+        if (tx >= 0 && ty >= 0 && tx < nx && ty < ny) still = still && __ldg(motion_max + ty * nx + tx) < kTaaStill;
+    }
+    still = __all_sync(0xffffffffu, still);
     const float GR = 2.118033988749895f;
     const float iResx = 1.0f / (float)W, iResy = 1.0f / (float)H;
     float* o = out + 4 * (size_t)i;
     Centre c;
-    c.uvx = ((float)px + 0.5f) / (float)W;
-    c.uvy = ((float)py + 0.5f) / (float)H;
     float cl[4], ll[4];
     int mode = 0;  // 0 done, 1 disoccluded, 2 spiral
+    int here = 0;  // the centre's flags
     if (valid) {
-        Tap t;
-        tap(rec, W, H, c.uvx, c.uvy, &t);
-#pragma unroll
-        for (int k = 0; k < 3; k++) {
-            c.no[k] = t.no[k];
-            c.co[k] = t.co[k];
-        }
-#pragma unroll
-        for (int k = 0; k < 4; k++) c.ma[k] = t.ma[k];
-        c.de = t.de;
-        c.mo[0] = t.mo[0];
-        c.mo[1] = t.mo[1];
+        here = taa_centre(I, rec, px, py, c);
         tex4(I.light, W, H, c.uvx, c.uvy, cl);
         if (c.de == 1.0f) {
             o[0] = cl[0];
@@ -219,60 +402,12 @@ __global__ void __launch_bounds__(128) k_taa(const TaaIn I, const float4* __rest
             mode = (clampg(oux, 0.0f, 1.0f) != oux || clampg(ouy, 0.0f, 1.0f) != ouy) ? 1 : 2;
         }
     }
-    // disocclusion: the current frame's 19x19 neighbourhood only
-    unsigned dis = __ballot_sync(0xffffffffu, mode == 1);
-    if (dis != 0u && __popc(dis) <= kDisCoopMax) {
-        float4* sd = s_dis[wib];
-        while (dis) {
-            const int p = __ffs(dis) - 1;
-            dis &= dis - 1u;
-            Centre q;
-            q.uvx = __shfl_sync(0xffffffffu, c.uvx, p);
-            q.uvy = __shfl_sync(0xffffffffu, c.uvy, p);
-#pragma unroll
-            for (int k = 0; k < 3; k++) {
-                q.no[k] = __shfl_sync(0xffffffffu, c.no[k], p);
-                q.co[k] = __shfl_sync(0xffffffffu, c.co[k], p);
-            }
-#pragma unroll
-            for (int k = 0; k < 4; k++) q.ma[k] = __shfl_sync(0xffffffffu, c.ma[k], p);
-            q.de = __shfl_sync(0xffffffffu, c.de, p);
-            q.mo[0] = __shfl_sync(0xffffffffu, c.mo[0], p);
-            q.mo[1] = __shfl_sync(0xffffffffu, c.mo[1], p);
-            for (int t = lane; t < kDisTaps; t += 32) sd[t] = disocc_tap(rec, W, H, iResx, iResy, q, t / 19 - 9, t % 19 - 9);
-            __syncwarp();
-            float acc = 0.0f;
-            if (lane < 4) {
-                const float* f = reinterpret_cast<const float*>(sd) + lane;
-                for (int t = 0; t < kDisTaps; t++) acc += f[4 * t];
-            }
-            const float s0 = __shfl_sync(0xffffffffu, acc, 0), s1 = __shfl_sync(0xffffffffu, acc, 1);
-            const float s2 = __shfl_sync(0xffffffffu, acc, 2), count = __shfl_sync(0xffffffffu, acc, 3);
-            if (lane == p) {
-                o[0] = s0 / count;
-                o[1] = s1 / count;
-                o[2] = s2 / count;
-                o[3] = 1.0f;
-            }
-            __syncwarp();
-        }
-        if (mode == 1) mode = 0;
-    }
-    if (mode == 1) {
-        float count = 0.0f, s0 = 0.0f, s1 = 0.0f, s2 = 0.0f;
-        for (int x = -9; x <= 9; ++x)
-            for (int y = -9; y <= 9; ++y) {
-                const float4 r = disocc_tap(rec, W, H, iResx, iResy, c, x, y);
-                s0 += r.x;
-                s1 += r.y;
-                s2 += r.z;
-                count += r.w;
-            }
-        o[0] = s0 / count;
-        o[1] = s1 / count;
-        o[2] = s2 / count;
-        o[3] = 1.0f;
-        return;
+    const unsigned dis = __ballot_sync(0xffffffffu, mode == 1);
+    if (dis != 0u) {
+        int at = 0;
+        if (lane == 0) at = atomicAdd(list, __popc(dis));
+        at = __shfl_sync(0xffffffffu, at, 0);
+        if (mode == 1) list[1 + at + __popc(dis & ((1u << lane) - 1u))] = i;
     }
     if (mode != 2) return;
     const float* motion = c.mo;
@@ -290,23 +425,56 @@ __global__ void __launch_bounds__(128) k_taa(const TaaIn I, const float4* __rest
     const float size = 12.0f;
     float radius = 1.0f;
     const float dscale = gmin(gmax(0.1f, 0.5f), 1.0f / depth);
+    const bool near = still && fabsf((size + 1.0f) * (lastVariance + 1.0f) * dscale) < kTaaReach;
     const float n0 = __ldg(I.noise + 4 * (size_t)i);
-    for (float angle = n0 * 3.1415f * GR; radius <= size; angle += 2.39f) {
+    float angle = n0 * 3.1415f * GR;
+    for (int k12 = 0; k12 < 12; k12++, angle += 2.39f) {
         radius += 1.0f;
         float sn, cs;
         sincos_own(angle, &sn, &cs);
         const float rv = radius * (lastVariance + 1.0f);
         const float ox = cs * iResx * rv * dscale, oy = sn * iResy * rv * dscale;
         const float u = clampg(uvx + ox, 0.001f, 0.999f), v = clampg(uvy + oy, 0.001f, 0.999f);
-        Tap t;
-        tap(rec, W, H, u, v, &t);
-        const float* nli = t.li;
-        float factor = 1.212f - radius / size;
-        factor *= glsl_step(0.8f, 1.0f - len4(cm, t.ma));
-        factor *= gmax(dot3(cn, t.no), 0.0f);
-        factor *= 1.0f - clampg(fabsf(depth - t.de) * FAR, 0.0f, 1.0f);
-        factor *= 1.0f - clampg(len3(cc, t.co) * 10000.0f, 0.0f, 1.0f);
-        if (len2(motion[0] - t.mo[0], motion[1] - t.mo[1]) > 0.1f) factor = 0.0f;
+        const TapAt t(W, H, u, v);
+        float ld[4], co[4];
+        t.get(rec, __ldg(rec + t.i00), false, ld);
+        const float4 c00 = __ldg(rec + n + t.i00);
+        const int f = __float_as_int(c00.w);
+        t.get(rec + n, c00, f & kTaaColor, co);
+        const float* nli = ld;
+        const float apart = len3(cc, co) * 10000.0f;
+        float factor = 0.0f;
+        if (!(apart >= 1.0f) || ((f | here) & kTaaWild)) {
+            float like = 1.0f, facing;
+            const int axis = (f >> kTaaNormal) & 7;
+            const bool wild = (f | here) & kTaaWild;
+            // materials of one bin per channel lie within 0.04 of one another
+            if (wild || ((f ^ here) >> kTaaMaterial) != 0 || (f & kTaaOdd)) {
+                float ma[4];
+                t.get(mat, __ldg(mat + t.i00), f & kTaaSurface, ma);
+                like = glsl_step(0.8f, 1.0f - len4(cm, ma));
+            }
+            if (wild || !(f & kTaaSurface) || axis == kTaaOther) {
+                float no[4];
+                t.get(rec + 2 * n, __ldg(rec + 2 * n + t.i00), f & kTaaSurface, no);
+                facing = dot3(cn, no);
+            } else {
+                // an axis interpolated with itself: its one component, and zeros
+                const float w = t.bx + t.ax;
+                const float c1 = axis < 2 ? cn[0] : (axis < 4 ? cn[1] : cn[2]);
+                facing = c1 * ((axis & 1) ? -(w * t.by + w * t.ay) : w * t.by + w * t.ay);
+            }
+            factor = c_ring[k12];
+            factor *= like;
+            factor *= gmax(facing, 0.0f);
+            factor *= 1.0f - clampg(fabsf(depth - ld[3]) * FAR, 0.0f, 1.0f);
+            factor *= 1.0f - clampg(apart, 0.0f, 1.0f);
+            if (!near) {
+                float mo[2];
+                t.motion(I.motion, mo);
+                if (len2(motion[0] - mo[0], motion[1] - mo[1]) > 0.1f) factor = 0.0f;
+            }
+        }
 #pragma unroll
         for (int k = 0; k < 3; k++) {
             nmin[k] = gmin(nmin[k], nli[k]);
@@ -345,13 +513,19 @@ vxl_status launch_light_taa(vxl_ctx* ctx, const vxl_taa_frame* f, float* out, cu
     TaaIn I{f->light, f->last_light, f->color, f->normal, f->material, f->depth, f->motion, f->noise, f->width,
             f->height};
     const size_t n = (size_t)f->width * f->height;
-    VXL_TRY(ctx_grow(&ctx->d_taa, &ctx->taa_bytes, n * kTaaPlanes * sizeof(float4)));
+    const dim3 pack((unsigned)((f->width + kPackW - 1) / kPackW), (unsigned)((f->height + kPackH - 1) / kPackH));
+    // planes, the pre-pass's maxima, and the list of disoccluded pixels (its length first)
+    const size_t planes = n * kTaaPlanes * sizeof(float4), maxima = (size_t)pack.x * pack.y * sizeof(float);
+    VXL_TRY(ctx_grow(&ctx->d_taa, &ctx->taa_bytes, planes + maxima + (n + 1) * sizeof(int)));
     float4* rec = (float4*)ctx->d_taa;
-    const unsigned pack_blocks = (unsigned)std::min<size_t>((n + 255) / 256, (size_t)ctx->sm_count * 8);
-    k_taa_pack<<<pack_blocks, 256, 0, s>>>(I, rec);
+    float* motion_max = (float*)((char*)ctx->d_taa + planes);
+    int* list = (int*)((char*)ctx->d_taa + planes + maxima);
+    k_taa_pack<<<pack, kPackW * kPackH, 0, s>>>(I, rec, motion_max, list);
     ctx->launches++;
-    const dim3 grid((unsigned)((f->width + 31) / 32), (unsigned)((f->height + 3) / 4));
-    k_taa<<<grid, 128, 0, s>>>(I, rec, out);
+    const dim3 grid((unsigned)((f->width + 31) / 32), (unsigned)((f->height + kTaaRows - 1) / kTaaRows));
+    k_taa<<<grid, 32 * kTaaRows, 0, s>>>(I, rec, motion_max, list, out);
+    ctx->launches++;
+    k_taa_edge<<<(unsigned)std::min<size_t>(n, (size_t)ctx->sm_count * 8), 128, 0, s>>>(I, rec, list, out);
     ctx->launches++;
     VXL_TRY_CUDA(cudaGetLastError());
     return VXL_OK;
