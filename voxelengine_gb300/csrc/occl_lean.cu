@@ -1076,6 +1076,30 @@ bool occl_lean_supported(const vxl_grid* g, const vxl_outputs* out, const vxl_tu
     return g->tl_words != nullptr && !out->records && tune.leap != 1 && !(g->tl_wide && tune.leap == 3);
 }
 
+// Smaller tiles for frames that would leave warps without one: a tile's rays
+// run one after another on its warp, so few large tiles are a long chain on a
+// part of the GPU, while large frames want large pools. Each halving is taken
+// where it measured faster (us, 10 rays a pixel on 128^3 / on a 1024^3 terrain,
+// tiles of 2, 4, 8, 16 pixels):
+//     4,000 pixels    33  36  43  63    /   57  62  69  121
+//    14,651 pixels    45  40  45  66    /   87  71  71  122
+//    40,000 pixels    77  63  53  72    /  172 119  93  130
+//   160,000 pixels   225 154 119 122    /  567 338 220  257
+//   320,000 pixels   430 286 211 188    / 1090 632 387  380
+// and only while a pool keeps 32 rays (with 2 rays a pixel and 80,000 pixels,
+// 46 us in tiles of 8, 38 in tiles of 16). Runs of pixels only: a tuned block
+// shape stays.
+static void small_frame_tiles(const vxl_ctx* ctx, int64_t npix, int R, vxl_tuning& t) {
+    if (t.kstep != 8 || t.grab != 1 || t.tile_w != t.tile_px || t.tile_px > 16) return;
+    const int64_t warps = (int64_t)ctx->sm_count * 32;
+    while (t.tile_px > 2 && t.tile_px / 2 * R >= 32) {
+        // tiles per warp below which the half is faster: 2.5 for 16, 0.75 for 8, 0.4 for 4
+        const int64_t pct = t.tile_px == 16 ? 250 : (t.tile_px == 8 ? 75 : 40);
+        if (npix * 100 >= warps * t.tile_px * pct) break;
+        t.tile_px = t.tile_w = t.tile_px / 2;
+    }
+}
+
 vxl_status launch_trace_occlusion_lean(vxl_ctx* ctx, const vxl_grid* g, const vxl_gbuffer* gb,
                                        const vxl_trace_params* p, const vxl_outputs* out,
                                        unsigned long long* d_counter, const vxl_tuning& tune, cudaStream_t s,
@@ -1087,12 +1111,15 @@ vxl_status launch_trace_occlusion_lean(vxl_ctx* ctx, const vxl_grid* g, const vx
         t.tile_px = 8;
         t.tile_w = 8;
     }
+    small_frame_tiles(ctx, gb->npix, R, t);
     if (g->tl_wide) {
         LeanSceneW PW;
         PW.S = scene_of(g, gb, p, out, t);
         PW.S.pix_base = pix_base;
         PW.L = lean_grid_w_of(g);
         VXL_TRY_CUDA(cudaMemsetAsync(d_counter, 0, sizeof(unsigned long long), s));
+        if (t.tile_px == 2) return launch_lean_w<2>(ctx, PW, d_counter, t.grab, s);
+        if (t.tile_px == 4) return launch_lean_w<4>(ctx, PW, d_counter, t.grab, s);
         if (t.tile_px == 8) return launch_lean_w<8>(ctx, PW, d_counter, t.grab, s);
         if (t.tile_px == 32) return launch_lean_w<32>(ctx, PW, d_counter, t.grab, s);
         return launch_lean_w<16>(ctx, PW, d_counter, t.grab, s);
@@ -1102,6 +1129,8 @@ vxl_status launch_trace_occlusion_lean(vxl_ctx* ctx, const vxl_grid* g, const vx
     P.S.pix_base = pix_base;
     P.L = lean_grid_of(g);
     VXL_TRY_CUDA(cudaMemsetAsync(d_counter, 0, sizeof(unsigned long long), s));
+    if (t.tile_px == 2) return launch_lean_t<2, 8>(ctx, P, d_counter, t.grab, s);
+    if (t.tile_px == 4) return launch_lean_t<4, 8>(ctx, P, d_counter, t.grab, s);
     if (t.tile_px == 8) return launch_lean_k<8>(ctx, P, d_counter, t, s);
     if (t.tile_px == 32) return launch_lean_k<32>(ctx, P, d_counter, t, s);
     return launch_lean_k<16>(ctx, P, d_counter, t, s);
@@ -1118,7 +1147,7 @@ bool lean_batch_supported(const vxl_batch_item* items, int n, const vxl_tuning& 
 size_t lean_batch_desc_bytes() { return sizeof(LeanScene); }
 
 // the launch shape of a batch: 8-pixel tiles when the 16-pixel pools of its
-// largest ray count would hold the SM below 8 blocks
+// largest ray count would hold the SM below 8 blocks; smaller ones for few pixels in all
 vxl_tuning lean_batch_tuning(const vxl_ctx* ctx, const vxl_batch_item* items, int n, const vxl_tuning& tune) {
     int mr = 1;
     for (int i = 0; i < n; i++)
@@ -1128,6 +1157,9 @@ vxl_tuning lean_batch_tuning(const vxl_ctx* ctx, const vxl_batch_item* items, in
         t.tile_px = 8;
         t.tile_w = 8;
     }
+    int64_t npix = 0;
+    for (int i = 0; i < n; i++) npix += items[i].gbuf.npix;
+    small_frame_tiles(ctx, npix, mr, t);
     return t;
 }
 
@@ -1208,6 +1240,8 @@ vxl_status launch_lean_batch(vxl_ctx* ctx, void* d_table, const void* h_table, i
     VXL_TRY_CUDA(cudaMemsetAsync(d_counter, 0, sizeof(unsigned long long), s));
     const LeanScene* tab = (const LeanScene*)d_table;
     const LeanScene* htab = (const LeanScene*)h_table;
+    if (t.tile_px == 2) return launch_lean_batch_k<2>(ctx, tab, htab, n, max_r, total_tiles, d_counter, t, s);
+    if (t.tile_px == 4) return launch_lean_batch_k<4>(ctx, tab, htab, n, max_r, total_tiles, d_counter, t, s);
     if (t.tile_px == 8) return launch_lean_batch_k<8>(ctx, tab, htab, n, max_r, total_tiles, d_counter, t, s);
     if (t.tile_px == 32) return launch_lean_batch_k<32>(ctx, tab, htab, n, max_r, total_tiles, d_counter, t, s);
     return launch_lean_batch_k<16>(ctx, tab, htab, n, max_r, total_tiles, d_counter, t, s);
