@@ -55,11 +55,10 @@ __global__ void __launch_bounds__(kVoxThreads) k_voxelize_na(GridView g, unsigne
     const int ii = first + (int)blockIdx.y;
     const DevInstance& I = inst[ii];
     const DevModel M = models[I.model];
-    const VoxTileShape S = vox_tile_shape(M.sx);
-    auto up = [](int v, int l) { return ((uint32_t)v + (1u << l) - 1u) >> l; };
-    if ((uint64_t)blockIdx.x >= (uint64_t)up(M.sx, S.lx) * up(M.sy, S.ly) * up(M.sz, S.lz)) return;  // whole blocks
+    const VoxTileAt at(M, blockIdx.x);
+    if (at.z >= vox_tiles(M.sz, at.S.lz)) return;  // whole blocks
     voxel_tile_init(sh);
-    voxel_tile(g, words, I.m, M, blockIdx.x, value != 0, aabb ? aabb + 6 * (size_t)ii : nullptr, sh);
+    voxel_tile(g, words, I.m, M, at, value != 0, aabb ? aabb + 6 * (size_t)ii : nullptr, sh);
 }
 
 cudaError_t launch_derive_view(const GridView& v, const TraceLayout& t, uint32_t* mask, int by, int bz, int tz,

@@ -13,7 +13,7 @@ namespace vxl {
 
 // Every block takes an equal run of the level's tiles: one search for the job
 // of its first tile, then it walks on.
-__global__ void __launch_bounds__(kVoxThreads) k_voxelize(GridView g, unsigned long long* words,
+__global__ void __launch_bounds__(kVoxThreads, 12) k_voxelize(GridView g, unsigned long long* words,
                                                           const VoxJob* __restrict__ jobs,
                                                           const uint64_t* __restrict__ first,
                                                           const DevModel* __restrict__ models, int job0, int job1,
@@ -32,11 +32,14 @@ __global__ void __launch_bounds__(kVoxThreads) k_voxelize(GridView g, unsigned l
             hi = mid - 1;
     }
     voxel_tile_init(sh);
-    for (; k < end; k++) {
+    while (k < end) {
         while (first[lo + 1] <= k) lo++;
         const VoxJob& J = jobs[lo];
         const DevModel M = models[J.model];
-        voxel_tile(g, words, J.m, M, (uint32_t)(k - first[lo]), J.op != 0, aabb ? aabb + 6 * (size_t)J.index : nullptr, sh);
+        const uint64_t stop = first[lo + 1] < end ? first[lo + 1] : end;
+        VoxTileAt at(M, (uint32_t)(k - first[lo]));
+        for (; k < stop; k++, at.next())
+            voxel_tile(g, words, J.m, M, at, J.op != 0, aabb ? aabb + 6 * (size_t)J.index : nullptr, sh);
     }
 }
 

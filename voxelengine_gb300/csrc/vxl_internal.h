@@ -223,23 +223,45 @@ struct VoxJob {
 vxl_status launch_voxelize_level(vxl_grid* g, const VoxJob* d_jobs, const uint64_t* d_first, const DevModel* d_models,
                                  int job0, int job1, uint64_t ntiles, int32_t* d_aabb, cudaStream_t s);
 
-// The voxelizer's tiles: 2^lx x 2^ly x 2^lz source voxels, 1024 of them, as
-// near a cube as lets a warp read runs of x (its image then covers few
-// bricks); narrow models take narrow tiles, which would otherwise be half
-// empty.
+// The voxelizer's tiles: 2^lx x 2^ly x 2^lz source voxels, 1024 of them, near
+// a cube (its image then covers few bricks). Of these shapes a model takes the
+// one that covers it with the fewest tiles, the first of equals: the voxels of
+// a model of 8 to 64 a side are 80% of its tiles' on average, 70% with
+// 16 x 8 x 8 alone.
 struct VoxTileShape {
     int lx, ly, lz;
 };
 #ifdef __CUDACC__
 __host__ __device__
 #endif
-inline VoxTileShape vox_tile_shape(int sx) {
-    return sx > 8 ? VoxTileShape{4, 3, 3} : (sx > 4 ? VoxTileShape{3, 4, 3} : VoxTileShape{2, 4, 4});
+inline uint32_t vox_tiles(int n, int l) {
+    return ((uint32_t)n + (1u << l) - 1u) >> l;
+}
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+inline VoxTileShape vox_tile_shape(int sx, int sy, int sz) {
+    // (lx, ly, lz), 3 bits each; lx + ly <= 7
+    constexpr uint32_t shapes[6] = {4 | 3 << 3 | 3 << 6, 3 | 4 << 3 | 3 << 6, 3 | 3 << 3 | 4 << 6,
+                                    5 | 2 << 3 | 3 << 6, 4 | 2 << 3 | 4 << 6, 2 | 4 << 3 | 4 << 6};
+    VoxTileShape best{4, 3, 3};
+    uint32_t least = 0xffffffffu;
+#ifdef __CUDACC__
+#pragma unroll
+#endif
+    for (int k = 0; k < 6; k++) {
+        const int lx = (int)(shapes[k] & 7u), ly = (int)(shapes[k] >> 3 & 7u), lz = (int)(shapes[k] >> 6);
+        const uint32_t n = vox_tiles(sx, lx) * vox_tiles(sy, ly) * vox_tiles(sz, lz);  // below 2^31: a model has at most 2^30 voxels
+        if (n < least) {
+            least = n;
+            best = VoxTileShape{lx, ly, lz};
+        }
+    }
+    return best;
 }
 inline uint64_t vox_tile_count(int sx, int sy, int sz) {
-    const VoxTileShape S = vox_tile_shape(sx);
-    auto up = [](int v, int l) { return ((uint64_t)v + (1u << l) - 1u) >> l; };
-    return up(sx, S.lx) * up(sy, S.ly) * up(sz, S.lz);
+    const VoxTileShape S = vox_tile_shape(sx, sy, sz);
+    return (uint64_t)vox_tiles(sx, S.lx) * vox_tiles(sy, S.ly) * vox_tiles(sz, S.lz);
 }
 
 }  // namespace vxl
