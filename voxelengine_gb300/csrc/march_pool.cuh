@@ -13,14 +13,16 @@
 //    each part runs its own loop;
 //  - floor() is one addition of a large constant that rounds down, whose low
 //    bits are the cell, and the mod(pos, 0.5) > 0.25 test of the fine part
-//    (Light.frag:142-148) is the difference of two such additions;
+//    (Light.frag:142-148) is the difference of two such additions; the word's
+//    address and the bit in it are sums of multiples of those, which run on
+//    the FMA pipe (in shifts and masks, on the ALU pipe: 2 to 6% slower);
 //  - positions are monotone, so one bounds test covers the four steps of a
 //    batch, and a ray outside the grid on the side it moves to is a miss at
 //    once (with records, its positions still advance to the last one).
-// Before -> after, at 1080p on a 512^3 grid: sun shadow + ambient 391 -> 237
-// us, reflection 364 -> 190 us, the pairs of 64 lights 287 -> 184 us; 1 M
-// incoherent sparse rays with records 271 -> 167 us. Still issue-bound (a test
-// is about 40 instructions).
+// Before -> after, at 1080p on a 512^3 grid: sun shadow + ambient 391 -> 226
+// us, reflection 364 -> 186 us, the pairs of 64 lights 287 -> 181 us; 1 M
+// incoherent sparse rays with records 271 -> 157 us. Still bound by the
+// instructions it issues (a fine test is about 37, a coarse one 22).
 #pragma once
 #include "vxl_device.cuh"
 
@@ -40,38 +42,56 @@ struct MarchPool {
 // id: the ray's index in the tile; kMarchSuper set for the SuperSparse marcher
 constexpr uint32_t kMarchSuper = 0x80000000u;
 
-// x + 1.5 * 2^(23 - k), rounded down, holds floor(2^k x) in its low bits (-2 < x < 2^20).
-// The shader's conversions truncate, so x in (-2, 0) reads block 0: floor() clamped to 0.
-constexpr float kFloor1 = 12582912.0f, kFloor2 = 6291456.0f, kFloor4 = 3145728.0f;
-constexpr uint32_t kFloor1Bits = 0x4B400000u, kFloor2Bits = 0x4AC00000u, kFloor4Bits = 0x4A400000u;
+// x + 1.5 * 2^(23 - k), rounded down, holds floor(2^k x) in its low bits
+// (|x| < 2^20): floor(x / 4), floor(x / 2) and floor(2 x) of a position.
+constexpr float kBrick = 50331648.0f, kBlock = 25165824.0f, kHalf = 6291456.0f;
+constexpr uint32_t kBrickBits = 0x4C400000u, kBlockBits = 0x4BC00000u;
 
-// bit of the fine part's cell: block (x/2, y/2, z/2), voxel by mod(pos, 0.5) > 0.25 per axis (-2 < pos < n)
-__device__ __forceinline__ bool march_fine_bit(const GridView& g, f3 p) {
-    uint32_t fx = __float_as_uint(__fadd_rd(p.x, kFloor2)), fy = __float_as_uint(__fadd_rd(p.y, kFloor2)),
-             fz = __float_as_uint(__fadd_rd(p.z, kFloor2));  // kFloor2Bits + floor(2x)
-    const uint32_t cx = __float_as_uint(__fadd_ru(p.x, kFloor4)), cy = __float_as_uint(__fadd_ru(p.y, kFloor4)),
-                   cz = __float_as_uint(__fadd_ru(p.z, kFloor4));  // kFloor4Bits + ceil(4x)
-    // ceil(4x) - 2 floor(2x) is 0, 1 or 2, and 2 exactly where frac(2x) > 0.5, i.e. mod(x, 0.5) > 0.25
-    const uint32_t q = (cx - 2u * fx) + 4u * (cy - 2u * fy) + 16u * (cz - 2u * fz) -
-                       21u * (kFloor4Bits - 2u * kFloor2Bits);
-    fx = max(fx, kFloor2Bits);
-    fy = max(fy, kFloor2Bits);
-    fz = max(fz, kFloor2Bits);
-    const uint32_t brick = (fx >> 3) + (fy >> 3) * (uint32_t)g.bx + (fz >> 3) * g.bxy -
-                           (kFloor2Bits >> 3) * (1u + (uint32_t)g.bx + g.bxy);
-    const uint32_t w = __ldg(reinterpret_cast<const uint32_t*>(g.words) + (2ull * brick + ((fz >> 2) & 1u)));
-    const uint32_t sh = ((q >> 1) & 0x15u) | ((fx >> 1) & 2u) | ((fy << 1) & 8u);
-    return (w >> sh) & 1u;
+// The 32 bits (half a brick) with the 2^3 block of position p (0 <= p < n) and
+// the block's first bit in them, modulo 32. Everything after the additions is
+// a sum of multiples of their bits, so it runs on the FMA pipe; the pipe of
+// shifts, masks and compares bounds this kernel.
+__device__ __forceinline__ uint32_t march_word(const GridView& g, f3 p, bool on, uint32_t* shift) {
+    const uint32_t bx = __float_as_uint(__fadd_rd(p.x, kBlock)), by = __float_as_uint(__fadd_rd(p.y, kBlock)),
+                   bz = __float_as_uint(__fadd_rd(p.z, kBlock));
+    const uint32_t wx = __float_as_uint(__fadd_rd(p.x, kBrick)), wy = __float_as_uint(__fadd_rd(p.y, kBrick)),
+                   wz = __float_as_uint(__fadd_rd(p.z, kBrick));
+    const uint32_t brick = wx + wy * (uint32_t)g.bx + wz * g.bxy - kBrickBits * (1u + (uint32_t)g.bx + g.bxy);
+    const uint32_t half = bz - 2u * wz - (kBlockBits - 2u * kBrickBits);
+    *shift = 2u * bx - 4u * wx + 8u * by - 16u * wy;  // the constants are multiples of 32
+    return on ? __ldg(reinterpret_cast<const uint32_t*>(g.words + brick) + half) : 0u;
 }
-// any voxel of the 2^3 block of the coarse part's cell (-2 < pos < n)
+// bit of the fine part's cell: its block's voxel by mod(pos, 0.5) > 0.25 per axis (Light.frag:142-148).
+// For x >= 0 that is ceil(2x - 0.5) - floor(2x): x - 0.25 is exact from 0.125 up, and below
+// both are 0 whatever its rounding.
+__device__ __forceinline__ bool march_fine_bit(const GridView& g, f3 p) {
+    const uint32_t fx = __float_as_uint(__fadd_rd(p.x, kHalf)), fy = __float_as_uint(__fadd_rd(p.y, kHalf)),
+                   fz = __float_as_uint(__fadd_rd(p.z, kHalf));
+    const uint32_t cx = __float_as_uint(__fadd_ru(p.x - 0.25f, kHalf)), cy = __float_as_uint(__fadd_ru(p.y - 0.25f, kHalf)),
+                   cz = __float_as_uint(__fadd_ru(p.z - 0.25f, kHalf));
+    uint32_t sh;
+    const uint32_t w = march_word(g, p, true, &sh);
+    sh += (cx - fx) + 4u * (cy - fy) + 16u * (cz - fz);
+    return __funnelshift_r(w, w, sh) & 1u;
+}
+// any voxel of the coarse part's block
 __device__ __forceinline__ bool march_coarse_bit(const GridView& g, f3 p) {
-    const uint32_t fx = max(__float_as_uint(__fadd_rd(p.x, kFloor1)), kFloor1Bits),
-                   fy = max(__float_as_uint(__fadd_rd(p.y, kFloor1)), kFloor1Bits),
-                   fz = max(__float_as_uint(__fadd_rd(p.z, kFloor1)), kFloor1Bits);  // kFloor1Bits + floor(x)
-    const uint32_t brick = (fx >> 2) + (fy >> 2) * (uint32_t)g.bx + (fz >> 2) * g.bxy -
-                           (kFloor1Bits >> 2) * (1u + (uint32_t)g.bx + g.bxy);
-    const uint32_t w = __ldg(reinterpret_cast<const uint32_t*>(g.words) + (2ull * brick + ((fz >> 1) & 1u)));
-    return ((w >> ((fx & 2u) | ((fy & 2u) << 2))) & 0x00330033u) != 0u;
+    uint32_t sh;
+    const uint32_t w = march_word(g, p, true, &sh);
+    return (__funnelshift_r(w, w, sh) & 0x00330033u) != 0u;
+}
+// Either test where p may lie below 0 (above -2: the shader's conversions
+// truncate, so such a coordinate reads block 0) or, with `on` false, anywhere.
+// Below 0 the shader's mod() rounds; this is its arithmetic.
+template <bool FINE>
+__device__ __forceinline__ bool march_bit(const GridView& g, f3 p, bool on) {
+    uint32_t sh;
+    const uint32_t w = march_word(g, mk(fmaxf(p.x, 0.0f), fmaxf(p.y, 0.0f), fmaxf(p.z, 0.0f)), on, &sh);
+    if (!FINE) return (__funnelshift_r(w, w, sh) & 0x00330033u) != 0u;
+    const bool qx = p.x - (__fadd_rd(p.x, kHalf) - kHalf) > 0.25f, qy = p.y - (__fadd_rd(p.y, kHalf) - kHalf) > 0.25f,
+               qz = p.z - (__fadd_rd(p.z, kHalf) - kHalf) > 0.25f;
+    sh += (qx ? 1u : 0u) + (qy ? 4u : 0u) + (qz ? 16u : 0u);
+    return __funnelshift_r(w, w, sh) & 1u;
 }
 // The tested voxel as the shader computes it.
 template <bool FINE>
@@ -86,7 +106,7 @@ __device__ __forceinline__ unsigned march_lanes_below() {
     return m;
 }
 
-// inside the cells that the shader reads; outside them it reads 0
+// inside the cells that the shader reads (see march_bit); outside them it reads 0
 __device__ __forceinline__ bool march_inside(const GridView& g, f3 p) {
     return p.x > -2.0f && p.y > -2.0f && p.z > -2.0f && p.x < (float)g.nx && p.y < (float)g.ny && p.z < (float)g.nz;
 }
@@ -105,31 +125,39 @@ __device__ __forceinline__ bool march_outside(const GridView& g, f3 p, f3 e) {
 }
 
 // The N tests from p on, s apart: bit j of the result set where test j finds a
-// voxel. q becomes the position after them. `in`: p is known to be inside (it
-// becomes so for q's batch); left: nothing can be hit from q on.
+// voxel. q becomes the position after them. `in`: p is known to lie in [0, n)
+// (it becomes so for q's batch); left: nothing can be hit from q on.
 template <bool FINE, int N>
 __device__ __forceinline__ unsigned march_tests(const GridView& g, f3 p, f3 s, f3& q, bool& in, bool skip, bool& left) {
     // where the last test lies, to far less than the half cell that the bounds leave
     const f3 e = mk(__fmaf_rn(s.x, (float)(N - 1), p.x), __fmaf_rn(s.y, (float)(N - 1), p.y),
                     __fmaf_rn(s.z, (float)(N - 1), p.z));
-    const bool in_e = e.x >= -1.5f && e.y >= -1.5f && e.z >= -1.5f && e.x <= (float)g.nx - 0.5f &&
+    const bool in_e = e.x >= 0.5f && e.y >= 0.5f && e.z >= 0.5f && e.x <= (float)g.nx - 0.5f &&
                       e.y <= (float)g.ny - 0.5f && e.z <= (float)g.nz - 0.5f;
     unsigned hits = 0u;
     q = p;
-    if (in && in_e) {  // every position from p to e is inside
+    const bool inner = in && in_e;  // every position from p to e is inside
+    const bool none = !inner && (skip || march_outside(g, p, e));
+    // One lane on the grid's edge sends its whole warp through the tests that
+    // look at every position: a branch per lane would run both loops.
+    if (__all_sync(__activemask(), inner || none)) {
+        if (inner) {
 #pragma unroll
-        for (int j = 0; j < N; j++) {
-            hits |= (FINE ? march_fine_bit(g, q) : march_coarse_bit(g, q)) ? 1u << j : 0u;
-            q = add(q, s);
+            for (int j = 0; j < N; j++) {
+                hits |= (FINE ? march_fine_bit(g, q) : march_coarse_bit(g, q)) ? 1u << j : 0u;
+                q = add(q, s);
+            }
+        } else {
+            for (int j = 0; j < N; j++) q = add(q, s);
+            left = march_gone(g, q, s);
         }
     } else {
-        const bool none = skip || march_outside(g, p, e);
 #pragma unroll 1
         for (int j = 0; j < N; j++) {
-            if (!none && march_inside(g, q)) hits |= (FINE ? march_fine_bit(g, q) : march_coarse_bit(g, q)) ? 1u << j : 0u;
+            hits |= march_bit<FINE>(g, q, !none && march_inside(g, q)) ? 1u << j : 0u;
             q = add(q, s);
         }
-        left = march_gone(g, q, s);
+        left = !inner && march_gone(g, q, s);
     }
     in = in_e;
     return hits;
@@ -167,7 +195,7 @@ __device__ __forceinline__ int march_part(const GridView& g, MarchPool& P, int c
                 ds = march_step0(id) * (FINE ? 1.0f : 2.0f);
                 d = FINE ? ds * (float)(kMarchFirst + 1) : march_dcoarse(id);
                 lim = FINE ? 16.0f : (dist < 164.0f ? dist : 164.0f);
-                in = march_inside(g, p);
+                in = p.x >= 0.0f && p.y >= 0.0f && p.z >= 0.0f && march_inside(g, p);
                 ghost = REC && march_gone(g, p, s);
                 busy = true;
             }
@@ -251,7 +279,7 @@ __device__ __forceinline__ void march_push(const GridView& g, MarchPool& P, int&
     const f3 s = mul(d, step0);
     f3 q = o;
     if (on) {
-        bool in = march_inside(g, o), left = false;
+        bool in = o.x >= 0.0f && o.y >= 0.0f && o.z >= 0.0f && march_inside(g, o), left = false;
         const unsigned hits = march_tests<true, kMarchFirst>(g, o, s, q, in, false, left);
         if (hits) {
             const int k = __ffs(hits) - 1;
