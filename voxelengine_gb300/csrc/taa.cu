@@ -18,7 +18,7 @@
 //    (flagged too: 0 times that is not 0);
 //  - the motion test (> 0.1 apart, :120) needs no loads where the pre-pass's
 //    per-tile maxima show that no tap in reach can fail it.
-// 1080p: 1171 + 37 us (every tap 16 16-byte loads) -> 459 + 130 + 41 us, about
+// 1080p: 1171 + 37 us (every tap 16 16-byte loads) -> 456 + 126 + 41 us, about
 // 60% issue-bound, the rest load latency.
 // Planes rather than records: the 16-byte loads of scattered taps then spread
 // over eight L1 bank groups (texel mod 8).
@@ -113,6 +113,7 @@ __global__ void __launch_bounds__(kPackW* kPackH) k_taa_pack(const TaaIn I, floa
     const int t0 = threadIdx.x, x0 = blockIdx.x * kPackW, y0 = blockIdx.y * kPackH;
     const size_t n = (size_t)I.W * I.H;
     float top = 0.0f;
+#pragma unroll
     for (int t = t0; t < SW * SH; t += kPackW * kPackH) {
         // texels of the block first, so that thread t0 holds texel t0 of the block
         const bool own = t < kPackW * kPackH;
@@ -241,31 +242,55 @@ struct Centre {
     float uvx, uvy, no[3], ma[4], de, co[3], mo[2];
 };
 
+// dot3 of the centre's normal with a tap's, and whether the materials are
+// alike (LightTAA.frag's step(0.8, 1 - distance)), with no loads where the
+// flags decide. f: the tap's flags, here: the centre's.
+__device__ __forceinline__ float taa_like(const float4* __restrict__ mat, const TapAt& t, const Centre& c, int f, int here) {
+    // materials of one bin per channel lie within 0.04 of one another
+    if (((f | here) & kTaaWild) == 0 && ((f ^ here) >> kTaaMaterial) == 0 && !(f & kTaaOdd)) return 1.0f;
+    float ma[4];
+    t.get(mat, __ldg(mat + t.i00), f & kTaaSurface, ma);
+    return glsl_step(0.8f, 1.0f - len4(c.ma, ma));
+}
+__device__ __forceinline__ float taa_facing(const float4* __restrict__ normals, const TapAt& t, const Centre& c, int f,
+                                            int here) {
+    const int axis = (f >> kTaaNormal) & 7;
+    if (((f | here) & kTaaWild) || !(f & kTaaSurface) || axis == kTaaOther) {
+        float no[4];
+        t.get(normals, __ldg(normals + t.i00), f & kTaaSurface, no);
+        return dot3(c.no, no);
+    }
+    // an axis interpolated with itself: its one component, and zeros
+    const float w = t.bx + t.ax;
+    const float c1 = axis < 2 ? c.no[0] : (axis < 4 ? c.no[1] : c.no[2]);
+    return c1 * ((axis & 1) ? -(w * t.by + w * t.ay) : w * t.by + w * t.ay);
+}
+
 // One tap (x, y) of the 19x19 disocclusion neighbourhood (LightTAA.frag:61-80):
 // (factor * light.rgb, factor), the terms its sums add in order.
 __device__ __forceinline__ float4 disocc_tap(const TaaIn& I, const float4* __restrict__ rec, float iResx, float iResy,
-                                             const Centre& c, bool wild, int x, int y) {
+                                             const Centre& c, int here, bool still, int x, int y) {
     const float FAR = 4096.0f;
     const float ox = (float)x * iResx, oy = (float)y * iResy;
     const float u = clampg(c.uvx + ox, 0.001f, 0.999f), v = clampg(c.uvy + oy, 0.001f, 0.999f);
     const TapAt t(I.W, I.H, u, v);
     const size_t n = (size_t)I.W * I.H;
-    const float4* mat = reinterpret_cast<const float4*>(I.material);
     const float4 c00 = __ldg(rec + n + t.i00);
     const int f = __float_as_int(c00.w);
-    float ld[4], co[4], no[4], ma[4], mo[2];
-    t.get(mat, __ldg(mat + t.i00), f & kTaaSurface, ma);
-    const float like = glsl_step(0.8f, 1.0f - len4(c.ma, ma));
-    if (like == 0.0f && !wild && !(f & kTaaWild)) return make_float4(0.0f, 0.0f, 0.0f, 0.0f);  // adds nothing
+    const float like = taa_like(reinterpret_cast<const float4*>(I.material), t, c, f, here);
+    if (like == 0.0f && !((f | here) & kTaaWild)) return make_float4(0.0f, 0.0f, 0.0f, 0.0f);  // adds nothing
+    float ld[4], co[4];
     t.get(rec, __ldg(rec + t.i00), false, ld);
     t.get(rec + n, c00, f & kTaaColor, co);
-    t.get(rec + 2 * n, __ldg(rec + 2 * n + t.i00), f & kTaaSurface, no);
-    t.motion(I.motion, mo);
-    float factor = gmax(dot3(c.no, no), 0.0f);
+    float factor = gmax(taa_facing(rec + 2 * n, t, c, f, here), 0.0f);
     factor *= like;
     factor *= 1.0f - clampg(fabsf(c.de - ld[3]) * FAR, 0.0f, 1.0f);
     factor *= 1.0f - clampg(len3(c.co, co), 0.0f, 1.0f);
-    if (len2(c.mo[0] - mo[0], c.mo[1] - mo[1]) > 0.1f) factor = 0.0f;
+    if (!still) {
+        float mo[2];
+        t.motion(I.motion, mo);
+        if (len2(c.mo[0] - mo[0], c.mo[1] - mo[1]) > 0.1f) factor = 0.0f;
+    }
     return make_float4(factor * ld[0], factor * ld[1], factor * ld[2], factor);
 }
 
@@ -276,7 +301,9 @@ __constant__ float c_ring[12] = {1.212f - 2.0f / 12.0f, 1.212f - 3.0f / 12.0f,  
 
 constexpr int kDisTaps = 19 * 19;
 
-// The centre of a pixel: everything its taps are compared with; returns its flags.
+// The centre of a pixel: everything its taps are compared with; returns its
+// flags. A warp's centres are neighbours, so all four texels are loaded at
+// once rather than the flags first.
 __device__ __forceinline__ int taa_centre(const TaaIn& I, const float4* __restrict__ rec, int px, int py, Centre& c) {
     const size_t n = (size_t)I.W * I.H;
     const float4* mat = reinterpret_cast<const float4*>(I.material);
@@ -286,19 +313,34 @@ __device__ __forceinline__ int taa_centre(const TaaIn& I, const float4* __restri
     float q[4];
     const float4 c00 = __ldg(rec + n + t.i00);
     const int f = __float_as_int(c00.w);
-    t.get(rec + n, c00, f & kTaaColor, q);
+    t.get(rec + n, c00, false, q);
     c.co[0] = q[0];
     c.co[1] = q[1];
     c.co[2] = q[2];
-    t.get(rec + 2 * n, __ldg(rec + 2 * n + t.i00), f & kTaaSurface, q);
+    t.get(rec + 2 * n, __ldg(rec + 2 * n + t.i00), false, q);
     c.no[0] = q[0];
     c.no[1] = q[1];
     c.no[2] = q[2];
-    t.get(mat, __ldg(mat + t.i00), f & kTaaSurface, c.ma);
+    t.get(mat, __ldg(mat + t.i00), false, c.ma);
     t.get(rec, __ldg(rec + t.i00), false, q);
     c.de = q[3];
     t.motion(I.motion, c.mo);
     return f;
+}
+
+// Reach of a pixel's taps, in texels, within which the motion test is decided
+// by the pre-pass's maxima: they lie at most 14.5 away, their texels at most
+// 16, so the block's own and its neighbouring tiles of 32 x 8 hold them, two
+// rows of tiles up and down. Motions below 0.035 differ by less than 0.1.
+constexpr float kTaaReach = 14.5f, kTaaStill = 0.035f;
+
+// By a whole warp: no tap in reach of a pixel of tile (tx, ty) can fail the motion test.
+__device__ __forceinline__ bool taa_still(int W, int H, int tx, int ty, const float* __restrict__ motion_max) {
+    const int lane = threadIdx.x & 31, nx = (W + kPackW - 1) / kPackW, ny = (H + kPackH - 1) / kPackH;
+    const int x = tx - 1 + lane % 3, y = ty - 2 + lane / 3;
+    bool still = W <= 14000 && H <= 14000;
+    if (lane < 15 && x >= 0 && y >= 0 && x < nx && y < ny) still = still && __ldg(motion_max + y * nx + x) < kTaaStill;
+    return __all_sync(0xffffffffu, still);
 }
 
 // The pixels whose reprojection leaves the screen (listed by k_taa), up to
@@ -308,13 +350,18 @@ __device__ __forceinline__ int taa_centre(const TaaIn& I, const float4* __restri
 // column by column, the shader's loop order, so the result is the same float.
 // 361 taps instead of 12: inside the spiral's kernel the few warps with such
 // pixels, at the screen's edge, ran on after all others (1080p, 1% of the
-// pixels: 958 us, now 459 for the spiral and 130 here).
+// pixels: 958 us, now 456 for the spiral and 126 here).
+// A block of 384 threads makes a pixel's taps in one go, for few pixels; many
+// run better in blocks of 128.
 constexpr int kEdgeGroup = 4;
-__global__ void __launch_bounds__(128) k_taa_edge(const TaaIn I, const float4* __restrict__ rec,
-                                                  const int* __restrict__ list, float* __restrict__ out) {
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS) k_taa_edge(const TaaIn I, const float4* __restrict__ rec,
+                                                  const float* __restrict__ motion_max, const int* __restrict__ list,
+                                                  float* __restrict__ out) {
     __shared__ float4 s_dis[kEdgeGroup][kDisTaps];
     __shared__ Centre s_centre[kEdgeGroup];
     __shared__ int s_flags[kEdgeGroup];
+    __shared__ bool s_still[kEdgeGroup];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const float iResx = 1.0f / (float)I.W, iResy = 1.0f / (float)I.H;
     const int count = list[0];
@@ -325,16 +372,18 @@ __global__ void __launch_bounds__(128) k_taa_edge(const TaaIn I, const float4* _
             const int i = list[1 + k + wib];
             Centre c;
             const int f = taa_centre(I, rec, i % I.W, i / I.W, c);
+            const bool still = taa_still(I.W, I.H, i % I.W / kPackW, i / I.W / kPackH, motion_max);
             if (lane == 0) {
+                s_still[wib] = still;
                 s_centre[wib] = c;
                 s_flags[wib] = f;
             }
         }
         __syncthreads();
         for (int e = 0; e < m; e++)
-            for (int t = threadIdx.x; t < kDisTaps; t += 128) {
+            for (int t = threadIdx.x; t < kDisTaps; t += THREADS) {
                 const int x = t % 19, y = t / 19;
-                s_dis[e][x * 19 + y] = disocc_tap(I, rec, iResx, iResy, s_centre[e], s_flags[e] & kTaaWild, x - 9, y - 9);
+                s_dis[e][x * 19 + y] = disocc_tap(I, rec, iResx, iResy, s_centre[e], s_flags[e], s_still[e], x - 9, y - 9);
             }
         __syncthreads();
         if (wib == 0) {
@@ -354,33 +403,25 @@ __global__ void __launch_bounds__(128) k_taa_edge(const TaaIn I, const float4* _
     }
 }
 
-// Reach of a pixel's taps, in texels, within which the motion test is decided
-// by the pre-pass's maxima: they lie at most 14.5 away, their texels at most
-// 16, so the block's own and its neighbouring tiles of 32 x 8 hold them, two
-// rows of tiles up and down. Motions below 0.035 differ by less than 0.1.
-constexpr float kTaaReach = 14.5f, kTaaStill = 0.035f;
-
 // 32x4-pixel blocks: the spiral taps of neighbouring pixels overlap in L1.
 // Four rows and 7 blocks per SM (72 registers, 48 bytes of spills) measured
-// 459 us at 1080p; 6 blocks 504, 8 blocks 484, two rows 484, eight rows 510.
+// 456 us at 1080p; 6 blocks 504, 8 blocks 484, two rows 484, eight rows 510.
 constexpr int kTaaRows = 4;
-__global__ void __launch_bounds__(32 * kTaaRows, 7) k_taa(const TaaIn I, const float4* __restrict__ rec,
-                                             const float* __restrict__ motion_max, int* __restrict__ list,
-                                                         float* __restrict__ out) {
+// SPLIT lanes share a pixel: lane s of them makes the taps s, s + SPLIT, ..,
+// and all add them up in the shader's order.
+template <int SPLIT, int BLOCKS>
+__global__ void __launch_bounds__(32 * kTaaRows, BLOCKS) k_taa(const TaaIn I, const float4* __restrict__ rec,
+                                                               const float* __restrict__ motion_max,
+                                                               int* __restrict__ list, float* __restrict__ out) {
+    constexpr int WIDE = 32 / SPLIT;  // pixels per warp
     const int W = I.W, H = I.H;
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    const int px = blockIdx.x * 32 + lane, py = blockIdx.y * kTaaRows + wib;
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, share = lane % SPLIT;
+    const int px = blockIdx.x * WIDE + lane / SPLIT, py = blockIdx.y * kTaaRows + wib;
     const bool valid = px < W && py < H;
     const int i = valid ? py * W + px : 0;
     const size_t n = (size_t)W * H;
     const float4* mat = reinterpret_cast<const float4*>(I.material);
-    bool still = W <= 14000 && H <= 14000;
-    if (lane < 15) {
-        const int tx = (int)blockIdx.x - 1 + lane % 3, ty = (int)(blockIdx.y * kTaaRows / kPackH) - 2 + lane / 3;
-        const int nx = (W + kPackW - 1) / kPackW, ny = (H + kPackH - 1) / kPackH;
-        if (tx >= 0 && ty >= 0 && tx < nx && ty < ny) still = still && __ldg(motion_max + ty * nx + tx) < kTaaStill;
-    }
-    still = __all_sync(0xffffffffu, still);
+    const bool still = taa_still(W, H, (int)(blockIdx.x * WIDE / kPackW), (int)(blockIdx.y * kTaaRows / kPackH), motion_max);
     const float GR = 2.118033988749895f;
     const float iResx = 1.0f / (float)W, iResy = 1.0f / (float)H;
     float* o = out + 4 * (size_t)i;
@@ -402,18 +443,16 @@ __global__ void __launch_bounds__(32 * kTaaRows, 7) k_taa(const TaaIn I, const f
             mode = (clampg(oux, 0.0f, 1.0f) != oux || clampg(ouy, 0.0f, 1.0f) != ouy) ? 1 : 2;
         }
     }
-    const unsigned dis = __ballot_sync(0xffffffffu, mode == 1);
+    const unsigned dis = __ballot_sync(0xffffffffu, mode == 1 && share == 0);
     if (dis != 0u) {
         int at = 0;
         if (lane == 0) at = atomicAdd(list, __popc(dis));
         at = __shfl_sync(0xffffffffu, at, 0);
-        if (mode == 1) list[1 + at + __popc(dis & ((1u << lane) - 1u))] = i;
+        if (mode == 1 && share == 0) list[1 + at + __popc(dis & ((1u << lane) - 1u))] = i;
     }
-    if (mode != 2) return;
+    if (mode != 2) return;  // with its pixel's other lanes
     const float* motion = c.mo;
     const float* cc = c.co;
-    const float* cm = c.ma;
-    const float* cn = c.no;
     const float depth = c.de;
     const float uvx = c.uvx, uvy = c.uvy;
     const float FAR = 4096.0f;
@@ -428,11 +467,23 @@ __global__ void __launch_bounds__(32 * kTaaRows, 7) k_taa(const TaaIn I, const f
     const bool near = still && fabsf((size + 1.0f) * (lastVariance + 1.0f) * dscale) < kTaaReach;
     const float n0 = __ldg(I.noise + 4 * (size_t)i);
     float angle = n0 * 3.1415f * GR;
-    for (int k12 = 0; k12 < 12; k12++, angle += 2.39f) {
-        radius += 1.0f;
+    // the pixel's lanes, which are all here
+    const unsigned group = SPLIT == 1 ? 1u << lane : ((1u << SPLIT) - 1u) << (lane - share);
+#pragma unroll 1
+    for (int k0 = 0; k0 < 12; k0 += SPLIT) {
+        float own = angle;  // of this lane's tap: the shader's sum, term by term
+        float rad = radius + 1.0f;
+        for (int j = 0; j < SPLIT; j++) {
+            if (j < share) {
+                own += 2.39f;
+                rad += 1.0f;
+            }
+            angle += 2.39f;
+            radius += 1.0f;
+        }
         float sn, cs;
-        sincos_own(angle, &sn, &cs);
-        const float rv = radius * (lastVariance + 1.0f);
+        sincos_own(own, &sn, &cs);
+        const float rv = rad * (lastVariance + 1.0f);
         const float ox = cs * iResx * rv * dscale, oy = sn * iResy * rv * dscale;
         const float u = clampg(uvx + ox, 0.001f, 0.999f), v = clampg(uvy + oy, 0.001f, 0.999f);
         const TapAt t(W, H, u, v);
@@ -441,32 +492,12 @@ __global__ void __launch_bounds__(32 * kTaaRows, 7) k_taa(const TaaIn I, const f
         const float4 c00 = __ldg(rec + n + t.i00);
         const int f = __float_as_int(c00.w);
         t.get(rec + n, c00, f & kTaaColor, co);
-        const float* nli = ld;
         const float apart = len3(cc, co) * 10000.0f;
         float factor = 0.0f;
         if (!(apart >= 1.0f) || ((f | here) & kTaaWild)) {
-            float like = 1.0f, facing;
-            const int axis = (f >> kTaaNormal) & 7;
-            const bool wild = (f | here) & kTaaWild;
-            // materials of one bin per channel lie within 0.04 of one another
-            if (wild || ((f ^ here) >> kTaaMaterial) != 0 || (f & kTaaOdd)) {
-                float ma[4];
-                t.get(mat, __ldg(mat + t.i00), f & kTaaSurface, ma);
-                like = glsl_step(0.8f, 1.0f - len4(cm, ma));
-            }
-            if (wild || !(f & kTaaSurface) || axis == kTaaOther) {
-                float no[4];
-                t.get(rec + 2 * n, __ldg(rec + 2 * n + t.i00), f & kTaaSurface, no);
-                facing = dot3(cn, no);
-            } else {
-                // an axis interpolated with itself: its one component, and zeros
-                const float w = t.bx + t.ax;
-                const float c1 = axis < 2 ? cn[0] : (axis < 4 ? cn[1] : cn[2]);
-                facing = c1 * ((axis & 1) ? -(w * t.by + w * t.ay) : w * t.by + w * t.ay);
-            }
-            factor = c_ring[k12];
-            factor *= like;
-            factor *= gmax(facing, 0.0f);
+            factor = c_ring[k0 + share];
+            factor *= taa_like(mat, t, c, f, here);
+            factor *= gmax(taa_facing(rec + 2 * n, t, c, f, here), 0.0f);
             factor *= 1.0f - clampg(fabsf(depth - ld[3]) * FAR, 0.0f, 1.0f);
             factor *= 1.0f - clampg(apart, 0.0f, 1.0f);
             if (!near) {
@@ -475,14 +506,26 @@ __global__ void __launch_bounds__(32 * kTaaRows, 7) k_taa(const TaaIn I, const f
                 if (len2(motion[0] - mo[0], motion[1] - mo[1]) > 0.1f) factor = 0.0f;
             }
         }
+        const float differ = len3(ld, cl) * factor;
 #pragma unroll
-        for (int k = 0; k < 3; k++) {
-            nmin[k] = gmin(nmin[k], nli[k]);
-            nmax[k] = gmax(nmax[k], nli[k]);
-            ncol[k] += factor * nli[k];
+        for (int j = 0; j < SPLIT; j++) {
+            float nli[3] = {ld[0], ld[1], ld[2]}, fj = factor, dj = differ;
+            if (SPLIT > 1) {
+                const int from = lane - share + j;
+#pragma unroll
+                for (int k = 0; k < 3; k++) nli[k] = __shfl_sync(group, ld[k], from);
+                fj = __shfl_sync(group, factor, from);
+                dj = __shfl_sync(group, differ, from);
+            }
+#pragma unroll
+            for (int k = 0; k < 3; k++) {
+                nmin[k] = gmin(nmin[k], nli[k]);
+                nmax[k] = gmax(nmax[k], nli[k]);
+                ncol[k] += fj * nli[k];
+            }
+            count += fj;
+            diffSum += dj;
         }
-        count += factor;
-        diffSum += len3(nli, cl) * factor;
     }
 #pragma unroll
     for (int k = 0; k < 3; k++) {
@@ -501,6 +544,7 @@ __global__ void __launch_bounds__(32 * kTaaRows, 7) k_taa(const TaaIn I, const f
     lastVariance += len2(motion[0], motion[1]) * 20.0f;
     const float t = clampg(1.0f - lastVariance, 0.3f, 0.9f);
     const float omt = 1.0f - t;
+    if (share != 0) return;
     o[0] = cl[0] * omt + ll[0] * t;
     o[1] = cl[1] * omt + ll[1] * t;
     o[2] = cl[2] * omt + ll[2] * t;
@@ -523,9 +567,23 @@ vxl_status launch_light_taa(vxl_ctx* ctx, const vxl_taa_frame* f, float* out, cu
     k_taa_pack<<<pack, kPackW * kPackH, 0, s>>>(I, rec, motion_max, list);
     ctx->launches++;
     const dim3 grid((unsigned)((f->width + 31) / 32), (unsigned)((f->height + kTaaRows - 1) / kTaaRows));
-    k_taa<<<grid, 32 * kTaaRows, 0, s>>>(I, rec, motion_max, list, out);
+    // A frame whose warps the GPU holds all at once takes as long as one pixel's
+    // 12 taps one after another: there four lanes share a pixel, and the edge
+    // runs in larger blocks (us, four lanes a pixel / one: 5,000 pixels 25 / 42,
+    // 40,000 38 / 47, 58,000 44 / 49, 80,000 54 / 54, 120,000 66 / 60).
+    const bool small = n <= (size_t)ctx->sm_count * 448;
+    if (small) {
+        const dim3 quarter((unsigned)((f->width + 7) / 8), grid.y);
+        k_taa<4, 7><<<quarter, 32 * kTaaRows, 0, s>>>(I, rec, motion_max, list, out);
+    } else {
+        k_taa<1, 7><<<grid, 32 * kTaaRows, 0, s>>>(I, rec, motion_max, list, out);
+    }
     ctx->launches++;
-    k_taa_edge<<<(unsigned)std::min<size_t>(n, (size_t)ctx->sm_count * 8), 128, 0, s>>>(I, rec, list, out);
+    const unsigned edge = (unsigned)std::min<size_t>(n, (size_t)ctx->sm_count * (small ? 2 : 8));
+    if (small)
+        k_taa_edge<384><<<edge, 384, 0, s>>>(I, rec, motion_max, list, out);
+    else
+        k_taa_edge<128><<<edge, 128, 0, s>>>(I, rec, motion_max, list, out);
     ctx->launches++;
     VXL_TRY_CUDA(cudaGetLastError());
     return VXL_OK;
