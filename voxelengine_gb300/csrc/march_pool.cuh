@@ -208,6 +208,13 @@ __device__ __forceinline__ int march_part(const GridView& g, MarchPool& P, int c
         bool run = busy, left = false;
         unsigned hits = 0u;
         do {
+            if (REC && run && ghost) {
+                // out of the grid for good: on to the last tests without looking
+                for (int b = 0; b < 8 && d + (float)N * ds < lim; b++) {
+                    for (int j = 0; j < N; j++) p = add(p, s);
+                    d = d + (float)N * ds;
+                }
+            }
             if (run) {
                 f3 q;
                 hits = march_tests<FINE, N>(g, p, s, q, in, REC && ghost, left);

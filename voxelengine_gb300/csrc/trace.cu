@@ -109,10 +109,19 @@ __global__ void __launch_bounds__(32 * kMarchWarps, kMarchBlocks)
     }
 }
 
-// The marchers: `tile` rays (a multiple of 32) per warp.
+// SuperSparse rays with records, one a thread: at most 29 tests a ray leave a
+// pool nothing to gain (400,000 rays from random points: 29 us, pooled 36).
+__global__ void __launch_bounds__(128) k_super_rays(GridView g, const float* __restrict__ rays, int64_t n,
+                                                    vxl_ray_record* __restrict__ rec) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const float* q = rays + 7 * i;
+        store_record(rec + i, march(g, mk(q[0], q[1], q[2]), mk(q[3], q[4], q[5]), q[6], 2.5f));
+    }
+}
+
+// Sparse rays with records: `tile` rays (a multiple of 32) per warp.
 __global__ void __launch_bounds__(32 * kMarchWarps, kMarchBlocks) k_march_rays(const __grid_constant__ GridView g,
-                                                                    const float* __restrict__ rays, int64_t n,
-                                                                    uint32_t super, int tile,
+                                                                    const float* __restrict__ rays, int64_t n, int tile,
                                                                     vxl_ray_record* __restrict__ rec) {
     __shared__ MarchPool pools[kMarchWarps];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -133,7 +142,7 @@ __global__ void __launch_bounds__(32 * kMarchWarps, kMarchBlocks) k_march_rays(c
             dist = q[6];
             if (!ray_domain_ok(o, d)) store_record(rec + i, Hit{0, 0, 0, dist, 0, 0});
         }
-        march_push<true>(g, P, count, i < n, o, d, dist, (uint32_t)k | super, done);
+        march_push<true>(g, P, count, i < n, o, d, dist, (uint32_t)k, done);
     }
     march_pool<true>(g, P, count, done);
 }
@@ -607,10 +616,11 @@ vxl_status launch_trace_rays(vxl_ctx* ctx, const vxl_grid* g, const float* rays,
         // grids beyond 64 MiB of words keep the brick in registers, as the occlusion pool does
         const unsigned b = (unsigned)std::min<int64_t>(march_blocks(n, 32), (int64_t)ctx->sm_count * kMarchBlocks);
         (g->nwords > (8ull << 20) ? k_trace_rays<true> : k_trace_rays<false>)<<<b, 32 * kMarchWarps, 0, s>>>(v, rays, n, rec);
-    } else {
+    } else if (mode == VXL_MODE_SPARSE) {
         const int tile = march_tile(ctx, n, 1);
-        k_march_rays<<<march_blocks(n, tile), 32 * kMarchWarps, 0, s>>>(v, rays, n, mode == VXL_MODE_SPARSE ? 0u : kMarchSuper,
-                                                                        tile, rec);
+        k_march_rays<<<march_blocks(n, tile), 32 * kMarchWarps, 0, s>>>(v, rays, n, tile, rec);
+    } else {
+        k_super_rays<<<grid_blocks(ctx, n, 128, 16), 128, 0, s>>>(v, rays, n, rec);
     }
     ctx->launches++;
     VXL_TRY_CUDA(cudaGetLastError());
