@@ -32,15 +32,15 @@ FORMS = {
 
 
 @pytest.mark.parametrize("form", sorted(FORMS))
-@pytest.mark.parametrize("n", [0, 1, 3])
+@pytest.mark.parametrize("n", [0, 1, 3, 9])
 def test_instance_table(form, n):
     ins = [(FORMS[form](k), k if k else np.int64(7), (1 << 32) + 1 if k == 2 else 1) for k in range(n)]
     assert bytes(V._instances(ins)) == bytes(_by_field(ins))
 
 
 def test_entity_table():
-    ents = [(M + k, FORMS["list"](k), (k, 0.1, -2), k) for k in range(3)]
-    arr = (V.Entity * 3)()
+    ents = [(M + k, FORMS["list"](k), (k, 0.1, -2), k) for k in range(7)]
+    arr = (V.Entity * 7)()
     for i, (pw, w, pv, mi) in enumerate(ents):
         arr[i].prev_world[:], arr[i].world[:] = [[float(x) for x in np.asarray(q, np.float32)] for q in (pw, w)]
         arr[i].pivot[:], arr[i].model = [float(x) for x in np.asarray(pv, np.float32)], mi
@@ -51,6 +51,6 @@ def test_entity_table():
 @pytest.mark.parametrize("bad", [(M[:15], 0, 1), (M, 1.0, 1), (M, 0), (M, 0, 1, 2), ("x", 0, 1), (M, "0", 1)])
 def test_refused(bad):
     for table in (_by_field, V._instances):
-        for ins in ([bad], [(M, 0, 1), bad], [bad, (M, 0, 1)]):
+        for ins in ([bad], [(M, 0, 1)] * 8 + [bad], [bad] + [(M, 0, 1)] * 8):
             with pytest.raises((TypeError, ValueError)):
                 table(ins)
