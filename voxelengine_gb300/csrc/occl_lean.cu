@@ -225,12 +225,12 @@ __device__ __forceinline__ int lean_batch(const uint32_t* __restrict__ w, uint32
     return stop;
 }
 
-// A warp refills its lanes when no more than this many run: the ends of rays
-// and the refill cost about as much as a batch, and taking them together at 26
-// is 1.2 to 1.8% faster than after every batch (512^3 at 1080p 1190 -> 1176 us, a mixed
-// batch 468 -> 462; 24 and 28 within 0.5%, 18: 1203). The wide layout's longer
-// rays gain 0.3% at 28 and lose below.
-constexpr int kLeanRefill = 26, kLeanRefillWide = 28;
+// The batched kernel's warps refill their lanes when no more than this many
+// run (DEFER): the ends of rays and the refill cost about as much as a batch,
+// and taking them together is 1.8% faster on a mix of 24 scenes (500.8 ->
+// 491.8 us; 24 and 28: 0.5% less). The single-scene kernel loses 0.2% at
+// 1080p on 512^3 with it and the wide layout 0.6%: they refill after every batch.
+constexpr int kLeanRefill = 26;
 
 #ifndef VXL_LEAN_MIN_BLOCKS
 #define VXL_LEAN_MIN_BLOCKS 8
@@ -240,7 +240,7 @@ constexpr int kLeanRefill = 26, kLeanRefillWide = 28;
 // traversal, fold (the phases of the pooled kernels in occlusion.cu). `one`
 // and `two27` (1 and 2^27) come from a kernel parameter at a fixed offset, so
 // the compiler can use them as constant operands rather than registers.
-template <int TP, int KSTEP>
+template <int TP, int KSTEP, bool DEFER>
 __device__ __forceinline__ void lean_tile(const SceneDesc& S, const LeanGrid& L, int64_t tile, PSlot* slots,
                                           float* res_t, uint32_t* res_hit, int lane, uint32_t one, uint32_t two27) {
     const TraceConstsP& c = S.c;
@@ -315,11 +315,83 @@ __device__ __forceinline__ void lean_tile(const SceneDesc& S, const LeanGrid& L,
 
     // ------------------------------------------------- B: traversal
     int base = 0;
-    bool busy = false;
+    bool busy = false, retired = false;
     uint32_t ax = 0, ay = 0, az = 0, kx = 0, ky = 0, kz = 0;
     float tx = 0.0f, ty = 0.0f, tz = 0.0f, tdx = 0.0f, tdy = 0.0f, tdz = 0.0f, maxt = 0.0f, tot = 0.0f;
     int n = 0, meta = 0;
-    for (;;) {
+    while (!DEFER) {
+        const bool need = !busy && !retired;
+        const unsigned nm = __ballot_sync(0xffffffffu, need);
+        if (nm) {
+            if (need) {
+                const int at = base + __popc(nm & lanes_below());
+                if (at < live) {
+                    const PSlot sl = slots[at];
+                    meta = (unsigned)sl.c2m >> 16;
+                    const int k = (meta >> 9) & 31;
+                    maxt = kind_maxt(c, k);
+                    {
+                        busy = true;
+                        const uint32_t A = (uint32_t)sl.c01;
+                        ax = A & L.field[0];
+                        ay = A & L.field[1];
+                        az = A & L.field[2];
+                        kx = (meta & 1) ? 0u - L.unit[0] : L.inc[0];
+                        ky = (meta & 2) ? 0u - L.unit[1] : L.inc[1];
+                        kz = (meta & 4) ? 0u - L.unit[2] : L.inc[2];
+                        tx = sl.a0; ty = sl.a1; tz = sl.a2;
+                        tdx = sl.b0; tdy = sl.b1; tdz = sl.b2;
+                        tot = -INFINITY;
+                        n = 0;
+                    }
+                } else {
+                    retired = true;
+                }
+            }
+            base += __popc(nm);
+        }
+        if (!__any_sync(0xffffffffu, busy) && base >= live) break;
+        if (busy) {
+            int res = 0;
+            float ht = 0.0f;
+            if (__all_sync(__activemask(), n + KSTEP <= 256)) {
+                const int st = lean_batch<KSTEP>(L.w, ax, ay, az, tx, ty, tz, tdx, tdy, tdz, kx, ky, kz,
+                                                 keep_y, keep_z, one, two27, maxt, tot);
+                if (st == 1)
+                    res = lean_set_cell(L, ax, ay, az, tx, ty, tz, tot, maxt, &ht) ? 1 : 2;
+                else if (st == 2)
+                    res = 2;
+                else {
+                    n += KSTEP;
+                    if (!(tot < maxt)) res = 2;
+                }
+            } else {
+                // the batch may reach the 256-iteration cap: test it, and maxt, at every iteration
+                for (int it = 0; it < KSTEP; it++) {
+                    if (n >= 256) {
+                        res = 2;
+                        break;
+                    }
+                    res = lean_step(L, ax, ay, az, tx, ty, tz, tdx, tdy, tdz, kx, ky, kz, maxt, tot, &ht);
+                    if (res) break;
+                    n++;
+                    if (!(tot < maxt) || n >= 256) {
+                        res = 2;
+                        break;
+                    }
+                }
+            }
+            if (res) {
+                if (res == 1) {
+                    const int k = (meta >> 9) & 31, pp = (meta >> 4) & 31;
+                    res_t[k * TP + pp] = ht;
+                    atomicOr(&res_hit[k], 1u << pp);
+                }
+                busy = false;
+            }
+        }
+    }
+    while (DEFER) {
         const unsigned idle = __ballot_sync(0xffffffffu, !busy);
         if (base < live) {
             const int at = base + __popc(idle & lanes_below());
@@ -461,7 +533,7 @@ __global__ void __launch_bounds__(128, VXL_LEAN_MIN_BLOCKS) k_occl_lean(const __
         t0 = __shfl_sync(0xffffffffu, t0, 0);
         if (t0 >= P.S.ntiles) break;
         for (int gi = 0; gi < grab && t0 + gi < P.S.ntiles; gi++)
-            lean_tile<TP, KSTEP>(P.S, P.L, t0 + gi, slots, res_t, res_hit, lane, P.L.one, P.L.two27);
+            lean_tile<TP, KSTEP, false>(P.S, P.L, t0 + gi, slots, res_t, res_hit, lane, P.L.one, P.L.two27);
     }
 }
 
@@ -510,7 +582,7 @@ __global__ void __launch_bounds__(128, VXL_LEAN_MIN_BLOCKS) k_occl_lean_batch(co
             PSlot* slots = reinterpret_cast<PSlot*>(wbase);
             float* res_t = reinterpret_cast<float*>(wbase + (size_t)TP * R * sizeof(PSlot));
             uint32_t* res_hit = reinterpret_cast<uint32_t*>(wbase + (size_t)TP * R * (sizeof(PSlot) + sizeof(float)));
-            lean_tile<TP, KSTEP>(desc->S, desc->L, t - cur_begin, slots, res_t, res_hit, lane, desc->L.one,
+            lean_tile<TP, KSTEP, true>(desc->S, desc->L, t - cur_begin, slots, res_t, res_hit, lane, desc->L.one,
                                  desc->L.two27);
         }
     }
@@ -575,7 +647,7 @@ __global__ void __launch_bounds__(128, VXL_LEAN_BATCH_MIN_BLOCKS) k_occl_lean_ba
             PSlot* slots = reinterpret_cast<PSlot*>(wbase);
             float* res_t = reinterpret_cast<float*>(wbase + (size_t)TP * R * sizeof(PSlot));
             uint32_t* res_hit = reinterpret_cast<uint32_t*>(wbase + (size_t)TP * R * (sizeof(PSlot) + sizeof(float)));
-            lean_tile<TP, KSTEP>(desc->S, desc->L, t - cur_begin, slots, res_t, res_hit, lane, one, two27);
+            lean_tile<TP, KSTEP, true>(desc->S, desc->L, t - cur_begin, slots, res_t, res_hit, lane, one, two27);
         }
     }
 }
@@ -906,80 +978,81 @@ __device__ __forceinline__ void lean_tile_w(const SceneDesc& S, const LeanGridW&
 
     // ------------------------------------------------- B: traversal
     int base = 0;
-    bool busy = false;
+    bool busy = false, retired = false;
     uint32_t ax = 0, ay = 0, kx = 0, ky = 0, wc = 0xffffffffu, wd = 0;
     uint64_t az = 0, kz = 0;
     float tx = 0.0f, ty = 0.0f, tz = 0.0f, tdx = 0.0f, tdy = 0.0f, tdz = 0.0f, maxt = 0.0f, tot = 0.0f;
     int n = 0, meta = 0;
     for (;;) {
-        const unsigned idle = __ballot_sync(0xffffffffu, !busy);
-        if (base < live) {
-            const int at = base + __popc(idle & lanes_below());
-            if (!busy && at < live) {
-                const PSlot sl = slots[at];
-                meta = (unsigned)sl.c2m >> 16;
-                const int k = (meta >> 9) & 31;
-                maxt = kind_maxt(c, k);
-                busy = true;
-                const uint64_t A = (uint64_t)(uint32_t)sl.c01 | ((uint64_t)(sl.c2m & 0xffff) << 32);
-                ax = (uint32_t)A & L.field[0];
-                ay = (uint32_t)A & L.field[1];
-                az = A & L.fieldz;
-                kx = (meta & 1) ? 0u - L.unit[0] : L.inc[0];
-                ky = (meta & 2) ? 0u - L.unit[1] : L.inc[1];
-                kz = (meta & 4) ? 0ull - L.unitz : L.incz;
-                tx = sl.a0; ty = sl.a1; tz = sl.a2;
-                tdx = sl.b0; tdy = sl.b1; tdz = sl.b2;
-                tot = -INFINITY;
-                n = 0;
-                wc = 0xffffffffu;
-            }
-            base += __popc(idle);
-        } else if (idle == 0xffffffffu) {
-            break;
-        }
-        const int waiting = base < live ? kLeanRefillWide : 0;
-        bool run = busy;
-        int end = 0;  // 1 set cell, 2 miss, 3 hit at ht
-        float ht = 0.0f;
-        do {
-            if (run) {
-                if (__all_sync(__activemask(), n + KSTEP <= 256)) {
-                    end = lean_batch_w(L.w, ax, ay, az, tx, ty, tz, tdx, tdy, tdz, kx, ky, (int32_t)kz, keep_y,
-                                                 keep_z, one, maxt, tot, wc, wd);
-                    if (end == 0) {
-                        n += KSTEP;
-                        if (!(tot < maxt)) end = 2;
+        const bool need = !busy && !retired;
+        const unsigned nm = __ballot_sync(0xffffffffu, need);
+        if (nm) {
+            if (need) {
+                const int at = base + __popc(nm & lanes_below());
+                if (at < live) {
+                    const PSlot sl = slots[at];
+                    meta = (unsigned)sl.c2m >> 16;
+                    const int k = (meta >> 9) & 31;
+                    maxt = kind_maxt(c, k);
+                    {
+                        busy = true;
+                        const uint64_t A = (uint64_t)(uint32_t)sl.c01 | ((uint64_t)(sl.c2m & 0xffff) << 32);
+                        ax = (uint32_t)A & L.field[0];
+                        ay = (uint32_t)A & L.field[1];
+                        az = A & L.fieldz;
+                        kx = (meta & 1) ? 0u - L.unit[0] : L.inc[0];
+                        ky = (meta & 2) ? 0u - L.unit[1] : L.inc[1];
+                        kz = (meta & 4) ? 0ull - L.unitz : L.incz;
+                        tx = sl.a0; ty = sl.a1; tz = sl.a2;
+                        tdx = sl.b0; tdy = sl.b1; tdz = sl.b2;
+                        tot = -INFINITY;
+                        n = 0;
+                        wc = 0xffffffffu;
                     }
                 } else {
-                    // the batch may reach the 256-iteration cap: test it, and maxt, at every iteration
-                    for (int it = 0; it < KSTEP; it++) {
-                        if (n >= 256) {
-                            end = 2;
-                            break;
-                        }
-                        const int res = lean_step_w(L, ax, ay, az, tx, ty, tz, tdx, tdy, tdz, kx, ky, kz, maxt, tot, &ht, wc, wd);
-                        if (res) {
-                            end = res == 1 ? 3 : 2;
-                            break;
-                        }
-                        n++;
-                        if (!(tot < maxt) || n >= 256) {
-                            end = 2;
-                            break;
-                        }
+                    retired = true;
+                }
+            }
+            base += __popc(nm);
+        }
+        if (!__any_sync(0xffffffffu, busy) && base >= live) break;
+        if (busy) {
+            int res = 0;
+            float ht = 0.0f;
+            if (__all_sync(__activemask(), n + KSTEP <= 256)) {
+                const int st = lean_batch_w(L.w, ax, ay, az, tx, ty, tz, tdx, tdy, tdz, kx, ky, (int32_t)kz, keep_y,
+                                            keep_z, one, maxt, tot, wc, wd);
+                if (st == 1)
+                    res = lean_set_cell_w(L, ax, ay, az, tx, ty, tz, tot, maxt, &ht) ? 1 : 2;
+                else if (st == 2)
+                    res = 2;
+                else {
+                    n += KSTEP;
+                    if (!(tot < maxt)) res = 2;
+                }
+            } else {
+                for (int it = 0; it < KSTEP; it++) {
+                    if (n >= 256) {
+                        res = 2;
+                        break;
+                    }
+                    res = lean_step_w(L, ax, ay, az, tx, ty, tz, tdx, tdy, tdz, kx, ky, kz, maxt, tot, &ht, wc, wd);
+                    if (res) break;
+                    n++;
+                    if (!(tot < maxt) || n >= 256) {
+                        res = 2;
+                        break;
                     }
                 }
-                run = end == 0;
             }
-        } while (__popc(__ballot_sync(0xffffffffu, run)) > waiting);
-        if (busy && !run) {
-            if (end == 3 || (end == 1 && lean_set_cell_w(L, ax, ay, az, tx, ty, tz, tot, maxt, &ht))) {
-                const int k = (meta >> 9) & 31, pp = (meta >> 4) & 31;
-                res_t[k * TP + pp] = ht;
-                atomicOr(&res_hit[k], 1u << pp);
+            if (res) {
+                if (res == 1) {
+                    const int k = (meta >> 9) & 31, pp = (meta >> 4) & 31;
+                    res_t[k * TP + pp] = ht;
+                    atomicOr(&res_hit[k], 1u << pp);
+                }
+                busy = false;
             }
-            busy = false;
         }
     }
     for (int i = lane; i < nlit; i += 32) {
