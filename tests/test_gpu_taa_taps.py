@@ -64,3 +64,16 @@ def test_negative_depth(vxl, ctx):
     fr = taa_cases.frame(W, H, 3, 0)
     fr["depth"][:] = -1e-3  # 1 / depth scales the spiral
     _check(vxl, ctx, fr, W, H)
+
+
+@pytest.mark.parametrize("W,H,band", [(400, 171, 0), (347, 199, 40), (1024, 70, 3)])
+def test_frames_of_one_lane_a_pixel(vxl, ctx, W, H, band):
+    """Above 68,096 pixels on this GPU (152 SMs): one lane a pixel, and the edge in blocks of 128, several pixels each
+    for the wide band."""
+    rng = np.random.default_rng(W)
+    fr = taa_cases.frame(W, H, W, band)
+    fr["motion"][H // 2:, W // 2:] *= np.float32(30.0)  # above the bound in a quarter of the frame
+    fr["last"][: H // 3, :, 3] = 3.0
+    for image, value in (("material", np.nan), ("depth", np.inf), ("color", -2e19), ("light", np.nan)):
+        fr[image][int(rng.integers(3, H)), int(rng.integers(0, W)), 0] = value
+    _check(vxl, ctx, fr, W, H)

@@ -10,8 +10,9 @@ from tests.gpu_util import dev, export_r8
 
 pytestmark = pytest.mark.gpu
 
-# (sx, sy, sz) around the three tile shapes 16x8x8, 8x16x8 and 4x16x16
-SHAPES = [(1, 1, 1), (1, 40, 3), (4, 16, 16), (4, 17, 33), (5, 16, 8), (8, 33, 9), (9, 8, 8), (16, 8, 8), (17, 9, 17), (48, 7, 25)]
+# (sx, sy, sz) around the tile shapes 16x8x8, 8x16x8, 8x8x16, 32x4x8, 16x4x16 and 4x16x16
+SHAPES = [(1, 1, 1), (1, 40, 3), (4, 16, 16), (4, 17, 33), (5, 16, 8), (8, 33, 9), (9, 8, 8), (16, 8, 8), (17, 9, 17), (48, 7, 25),
+          (8, 8, 16), (7, 8, 31), (32, 4, 8), (31, 3, 24), (64, 4, 9), (16, 4, 16), (15, 4, 32), (33, 12, 16)]
 
 
 def check(vxl, ctx, n, models, insts, noalloc=False):
