@@ -674,7 +674,8 @@ vxl_status launch_trace_primary(vxl_ctx* ctx, const vxl_volume* volumes, int nvo
     VXL_TRY_CUDA(cudaEventRecord(ctx->pev, s));
     const int64_t cap = (int64_t)ctx->plist_cap;
     if (n > 0) {
-        k_prim_fill<<<(unsigned)ctx->sm_count * 4, 256, 0, s>>>(d_ins, n, C.tiles_x, d_off, d_cur, ctx->d_plist, cap,
+        // the searches' loads are a chain: 8 blocks per SM 9 us, 4 blocks 11 (4096 instances at 1080p)
+        k_prim_fill<<<(unsigned)ctx->sm_count * 8, 256, 0, s>>>(d_ins, n, C.tiles_x, d_off, d_cur, ctx->d_plist, cap,
                                                                d_poff);
         ctx->launches++;
     }
