@@ -117,7 +117,14 @@ __device__ __forceinline__ bool march_gone(const GridView& g, f3 p, f3 s) {
            (p.z >= (float)g.nz && s.z >= 0.0f);
 }
 
-// All positions from p to about e lie outside, on the same side.
+// All positions from p to about e lie outside, on the same side. The half cell
+// covers the rounding of the positions and of e for steps below kMarchSlack: a
+// position near the grid is then at most 2^21 away from p and from the origin,
+// where the at most four roundings make 1/4 (at 2^24 a step, two cells).
+constexpr float kMarchSlack = 524288.0f;
+__device__ __forceinline__ bool march_small(f3 s) {
+    return fmaxf(fmaxf(fabsf(s.x), fabsf(s.y)), fabsf(s.z)) < kMarchSlack;
+}
 __device__ __forceinline__ bool march_outside(const GridView& g, f3 p, f3 e) {
     return fmaxf(p.x, e.x + 0.5f) <= -2.0f || fmaxf(p.y, e.y + 0.5f) <= -2.0f || fmaxf(p.z, e.z + 0.5f) <= -2.0f ||
            fminf(p.x, e.x - 0.5f) >= (float)g.nx || fminf(p.y, e.y - 0.5f) >= (float)g.ny ||
@@ -126,9 +133,11 @@ __device__ __forceinline__ bool march_outside(const GridView& g, f3 p, f3 e) {
 
 // The N tests from p on, s apart: bit j of the result set where test j finds a
 // voxel. q becomes the position after them. `in`: p is known to lie in [0, n)
-// (it becomes so for q's batch); left: nothing can be hit from q on.
+// (it becomes so for q's batch); skip: that nothing can be hit; small:
+// march_small(s); left: nothing can be hit from q on.
 template <bool FINE, int N>
-__device__ __forceinline__ unsigned march_tests(const GridView& g, f3 p, f3 s, f3& q, bool& in, bool skip, bool& left) {
+__device__ __forceinline__ unsigned march_tests(const GridView& g, f3 p, f3 s, f3& q, bool& in, bool skip, bool small,
+                                                bool& left) {
     // where the last test lies, to far less than the half cell that the bounds leave
     const f3 e = mk(__fmaf_rn(s.x, (float)(N - 1), p.x), __fmaf_rn(s.y, (float)(N - 1), p.y),
                     __fmaf_rn(s.z, (float)(N - 1), p.z));
@@ -137,7 +146,7 @@ __device__ __forceinline__ unsigned march_tests(const GridView& g, f3 p, f3 s, f
     unsigned hits = 0u;
     q = p;
     const bool inner = in && in_e;  // every position from p to e is inside
-    const bool none = !inner && (skip || march_outside(g, p, e));
+    const bool none = !inner && (skip || (small && march_outside(g, p, e)));
     // One lane on the grid's edge sends its whole warp through the tests that
     // look at every position: a branch per lane would run both loops.
     if (__all_sync(__activemask(), inner || none)) {
@@ -178,7 +187,7 @@ template <bool FINE, bool REC, class Done>
 __device__ __forceinline__ int march_part(const GridView& g, MarchPool& P, int count, Done done) {
     constexpr int N = kMarchBatch;
     int base = 0, kept = 0;
-    bool busy = false, in = false, ghost = false;
+    bool busy = false, in = false, ghost = false, small = true;
     f3 p = mk(0.0f, 0.0f, 0.0f), s = p;
     float d = 0.0f, ds = 0.0f, lim = 0.0f, dist = 0.0f;
     uint32_t id = 0;
@@ -197,6 +206,7 @@ __device__ __forceinline__ int march_part(const GridView& g, MarchPool& P, int c
                 lim = FINE ? 16.0f : (dist < 164.0f ? dist : 164.0f);
                 in = p.x >= 0.0f && p.y >= 0.0f && p.z >= 0.0f && march_inside(g, p);
                 ghost = REC && march_gone(g, p, s);
+                small = march_small(s);
                 busy = true;
             }
             base = min(base + __popc(idle), count);
@@ -217,7 +227,7 @@ __device__ __forceinline__ int march_part(const GridView& g, MarchPool& P, int c
             }
             if (run) {
                 f3 q;
-                hits = march_tests<FINE, N>(g, p, s, q, in, REC && ghost, left);
+                hits = march_tests<FINE, N>(g, p, s, q, in, REC && ghost, small, left);
                 const float dn = d + (float)N * ds;  // small multiples of 0.5: exact
                 if (hits != 0u || !(dn < lim) || (left && !REC)) {
                     run = false;
@@ -287,7 +297,7 @@ __device__ __forceinline__ void march_push(const GridView& g, MarchPool& P, int&
     f3 q = o;
     if (on) {
         bool in = o.x >= 0.0f && o.y >= 0.0f && o.z >= 0.0f && march_inside(g, o), left = false;
-        const unsigned hits = march_tests<true, kMarchFirst>(g, o, s, q, in, false, left);
+        const unsigned hits = march_tests<true, kMarchFirst>(g, o, s, q, in, false, march_small(s), left);
         if (hits) {
             const int k = __ffs(hits) - 1;
             f3 p = o;
