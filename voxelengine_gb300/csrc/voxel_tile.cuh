@@ -110,8 +110,9 @@ __device__ __forceinline__ void voxel_tile(const GridView& g, unsigned long long
     // voxels go to the grid one by one
     const bool gather = some && (uint64_t)wx * wy * wz <= kVoxBricks;
     const uint32_t wxy = wx * wy;
-    // the whole image lies inside the grid (the usual tile): its voxels need no bounds
-    const bool inside = gather && !(__ballot_sync(0xffffffffu, clipped) & 63u);
+    // the whole image lies inside the grid (the usual tile): its voxels need no
+    // bounds, and z is counted up as a float, which holds whole numbers to 2^24
+    const bool inside = gather && z1 <= 1 << 24 && !(__ballot_sync(0xffffffffu, clipped) & 63u);
 
     // o = M[3], dx,dy,dz = M[0..2] * 0.1f; wp = o + x*dx + y*dy + z*dz; fwp = ivec3(wp * 10) (:137-147)
     const f3 dz = mk(m[8] * 0.1f, m[9] * 0.1f, m[10] * 0.1f);
