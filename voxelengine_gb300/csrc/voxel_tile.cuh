@@ -174,9 +174,10 @@ __device__ __forceinline__ void voxel_tile(const GridView& g, unsigned long long
 #pragma unroll
         for (int a = 0; a < 3; a++) {
             const int l = __reduce_min_sync(0xffffffffu, lo[a]), h = __reduce_max_sync(0xffffffffu, hi[a]);
-            if ((t & 31) == 0 && l != INT_MAX) {
-                atomicMin(&sh.lo[a], l);
-                atomicMax(&sh.hi[a], h);
+            // a cell can be INT_MAX or INT_MIN itself (conversions saturate), so each bound is its own test
+            if ((t & 31) == 0) {
+                if (l != INT_MAX) atomicMin(&sh.lo[a], l);
+                if (h != INT_MIN) atomicMax(&sh.hi[a], h);
             }
         }
     }
@@ -198,9 +199,9 @@ __device__ __forceinline__ void voxel_tile(const GridView& g, unsigned long long
                 atomicAnd(w, ~b);
         }
     }
-    if (aabb && threadIdx.x < 3 && sh.lo[threadIdx.x] != INT_MAX) {
-        atomicMin(aabb + threadIdx.x, sh.lo[threadIdx.x]);
-        atomicMax(aabb + 3 + threadIdx.x, sh.hi[threadIdx.x]);
+    if (aabb && threadIdx.x < 3) {
+        if (sh.lo[threadIdx.x] != INT_MAX) atomicMin(aabb + threadIdx.x, sh.lo[threadIdx.x]);
+        if (sh.hi[threadIdx.x] != INT_MIN) atomicMax(aabb + 3 + threadIdx.x, sh.hi[threadIdx.x]);
         sh.lo[threadIdx.x] = INT_MAX;
         sh.hi[threadIdx.x] = INT_MIN;
     }
