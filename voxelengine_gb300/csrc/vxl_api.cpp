@@ -233,15 +233,22 @@ static vxl_status voxelize_runs(vxl_ctx* ctx, vxl_grid* g, const vxl_model* mode
     char* base = (char*)scratch;
     VXL_TRY_CUDA(cudaMemcpyAsync(base, h, total, cudaMemcpyHostToDevice, s));
     if (h_aabb) d_aabb = (int32_t*)(base + o_box);
-    for (int l = 0; l < nlev; l++)
-        VXL_TRY(launch_voxelize_level(g, (const VoxJob*)base, (const uint64_t*)(base + o_first),
-                                      (const DevModel*)(base + o_mod), at[l], at[(size_t)l + 1],
-                                      first[at[(size_t)l + 1]] - first[at[l]], d_aabb, s));
-    if (h_aabb) VXL_TRY_CUDA(cudaMemcpyAsync(h + o_box, d_aabb, b_box, cudaMemcpyDeviceToHost, s));
-    VXL_TRY_CUDA(cudaEventRecord(ctx->vox_ev, s));
-    // the tile map and the trace layout are queued before the wait, so the GPU goes on with them meanwhile
-    VXL_TRY(launch_build_tile_mask(g, s));
-    VXL_TRY_CUDA(cudaEventSynchronize(ctx->vox_ev));
+    const vxl_status st = [&]() -> vxl_status {
+        for (int l = 0; l < nlev; l++)
+            VXL_TRY(launch_voxelize_level(g, (const VoxJob*)base, (const uint64_t*)(base + o_first),
+                                          (const DevModel*)(base + o_mod), at[l], at[(size_t)l + 1],
+                                          first[at[(size_t)l + 1]] - first[at[l]], d_aabb, s));
+        if (h_aabb) VXL_TRY_CUDA(cudaMemcpyAsync(h + o_box, d_aabb, b_box, cudaMemcpyDeviceToHost, s));
+        VXL_TRY_CUDA(cudaEventRecord(ctx->vox_ev, s));
+        // the tile map and the trace layout are queued before the wait, so the GPU goes on with them meanwhile
+        VXL_TRY(launch_build_tile_mask(g, s));
+        VXL_TRY_CUDA(cudaEventSynchronize(ctx->vox_ev));
+        return VXL_OK;
+    }();
+    if (st != VXL_OK) {
+        cudaStreamSynchronize(s);  // what was queued still reads the image, the scratch and the models
+        return st;
+    }
     if (h_aabb) std::memcpy(h_aabb, h + o_box, b_box);
     return VXL_OK;
 }
