@@ -93,9 +93,12 @@ vxl_status vxl_ctx_launch_count(const vxl_ctx* ctx, uint64_t* out);
 
 /* Launch-shape knobs of the occlusion kernel (results do not depend on them).
  * Zero fields keep the current value. Picked per device by the autotuner
- * (voxelengine_gb300/autotune.py). */
+ * (voxelengine_gb300/autotune.py). A tile shape set here is kept for frames of
+ * every size. On a new context, and after all six fields are set to what
+ * vxl_ctx_get_tuning returns there, small frames run smaller tiles (2, 4 or 8
+ * pixels) where those are faster. */
 typedef struct vxl_tuning {
-    int32_t tile_px;   /* pixels per warp tile: 8, 16 or 32 (the exact-step and batched kernels run 8 as 16) */
+    int32_t tile_px;   /* pixels per warp tile: 8, 16 or 32 (the exact-step kernels run 8 as 16) */
     int32_t kstep;     /* DDA iterations between pool refills: 1, 2, 4, 8 or 16 (16: the single-scene
                           trace-layout kernel; the others run 8 for it) */
     int32_t leap;      /* empty-space skipping: 1 = cross empty bricks in one step where exact; 2 = none;

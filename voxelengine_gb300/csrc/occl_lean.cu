@@ -1164,10 +1164,9 @@ bool occl_lean_supported(const vxl_grid* g, const vxl_outputs* out, const vxl_tu
 //   160,000 pixels   225 154 119 122    /  567 338 220  257
 //   320,000 pixels   430 286 211 188    / 1090 632 387  380
 // and only while a pool keeps 32 rays (with 2 rays a pixel and 80,000 pixels,
-// 46 us in tiles of 8, 38 in tiles of 16). Runs of pixels only: a tuned block
-// shape stays.
+// 46 us in tiles of 8, 38 in tiles of 16). A tile that the caller chose stays.
 static void small_frame_tiles(const vxl_ctx* ctx, int64_t npix, int R, vxl_tuning& t) {
-    if (t.kstep != 8 || t.grab != 1 || t.tile_w != t.tile_px || t.tile_px > 16) return;
+    if (ctx->tile_chosen || t.kstep != 8 || t.grab != 1 || t.tile_w != t.tile_px || t.tile_px > 16) return;
     const int64_t warps = (int64_t)ctx->sm_count * 32;
     while (t.tile_px > 2 && t.tile_px / 2 * R >= 32) {
         // tiles per warp below which the half is faster: 2.5 for 16, 0.75 for 8, 0.4 for 4

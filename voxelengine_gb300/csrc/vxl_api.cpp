@@ -335,7 +335,7 @@ vxl_status vxl_ctx_create(int device, vxl_ctx** out) {
         delete c;
         return cuda_fail(e, "ctx_create");
     }
-    c->tune = vxl_tuning{16, 8, 2, 1, 16, 1};  // best on GB300 for the 512^3 / 1080p workload
+    c->tune = kDefaultTuning;
     *out = c;
     return VXL_OK;
 }
@@ -401,6 +401,7 @@ vxl_status vxl_ctx_set_tuning(vxl_ctx* ctx, const vxl_tuning* t) {
     if (n.tile_w > n.tile_px || n.tile_px % n.tile_w != 0 ||
         (n.tile_w != n.tile_px && n.tile_w != 4 && n.tile_w != 8))
         n.tile_w = n.tile_px;  // shapes that do not divide the tile fall back to pixel runs
+    if (t->tile_px || t->tile_w) ctx->tile_chosen = std::memcmp(t, &kDefaultTuning, sizeof *t) != 0;
     ctx->tune = n;
     return VXL_OK;
 }

@@ -8,6 +8,9 @@
 
 #include "../../include/vxl.h"
 
+// launch shape of a new context: best on GB300 for 512^3 at 1080p
+constexpr vxl_tuning kDefaultTuning{16, 8, 2, 1, 16, 1};
+
 struct vxl_ctx {
     int device;
     int sm_count;
@@ -27,6 +30,7 @@ struct vxl_ctx {
     uint32_t counter_next;
     uint32_t capture_next;
     vxl_tuning tune;  // occlusion kernel launch shape (vxl_ctx_set_tuning)
+    bool tile_chosen;  // its tile is the caller's: kept for small frames too
     // copy / compute pipeline of the host-buffer entry point (created on first use)
     cudaStream_t pipe[2];
     cudaEvent_t pipe_start;
