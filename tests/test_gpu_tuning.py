@@ -10,7 +10,7 @@ pytestmark = pytest.mark.gpu
 KEYS = ("shadow", "ao", "ao_vis", "spec", "spec_t")
 
 
-def _items(vxl, ctx, sizes):
+def _items(vxl, ctx, sizes, n_ao=8):
     import torch
 
     items = []
@@ -20,7 +20,7 @@ def _items(vxl, ctx, sizes):
         cam, tgt = np.array([32, 62, -14], np.float32), np.array([32, 19, 28], np.float32)
         pos, nrm, rough = empty(W * H * 3, torch.float32), empty(W * H * 3, torch.float32), empty(W * H, torch.float32)
         vxl.scene_gbuffer(ctx, G, cam, tgt, W, H, i, pos, nrm, rough)
-        kw = dict(light_dir=(0.3, 0.8, 0.5), cam_pos=cam, n_ao=8, ao_len=24.0, n_spec=1, seed=i)
+        kw = dict(light_dir=(0.3, 0.8, 0.5), cam_pos=cam, n_ao=n_ao, ao_len=24.0, n_spec=1, seed=i)
         items.append(dict(grid=G, npix=W * H, width=W, height=H, params=vxl.make_params(**kw), pos=pos, nrm=nrm,
                           rough=rough, kw=kw, **{k: empty(W * H, torch.float32) for k in KEYS}))
     return items
@@ -69,4 +69,17 @@ def test_large_batches_run_16_pixels(vxl):
     ctx = vxl.Context(0)
     items = _items(vxl, ctx, [(417, 311), (401, 307), (3, 5)])
     assert _tiles(vxl, ctx, items) == sum(-(-it["npix"] // 16) for it in items)
+    _match(items)
+
+
+@pytest.mark.parametrize("n_ao,size,px", [(4, (251, 160), 8), (4, (400, 301), 16), (8, (251, 160), 8), (8, (400, 301), 8),
+                                          (16, (101, 50), 2)])
+def test_default_tiles(vxl, n_ao, size, px):
+    """The measured choice by pixels and rays a pixel, for the 152 SMs that it was measured on."""
+    import torch
+
+    if torch.cuda.get_device_properties(0).multi_processor_count != 152:
+        pytest.skip("measured on 152 SMs")
+    items = _items(vxl, ctx := vxl.Context(0), [size], n_ao)
+    assert _tiles(vxl, ctx, items) == -(-items[0]["npix"] // px)
     _match(items)

@@ -1155,22 +1155,31 @@ bool occl_lean_supported(const vxl_grid* g, const vxl_outputs* out, const vxl_tu
 
 // Smaller tiles for frames that would leave warps without one: a tile's rays
 // run one after another on its warp, so few large tiles are a long chain on a
-// part of the GPU, while large frames want large pools. Each halving is taken
-// where it measured faster (us, 10 rays a pixel on 128^3 / on a 1024^3 terrain,
-// tiles of 2, 4, 8, 16 pixels):
-//     4,000 pixels    33  36  43  63    /   57  62  69  121
-//    14,651 pixels    45  40  45  66    /   87  71  71  122
-//    40,000 pixels    77  63  53  72    /  172 119  93  130
-//   160,000 pixels   225 154 119 122    /  567 338 220  257
-//   320,000 pixels   430 286 211 188    / 1090 632 387  380
-// and only while a pool keeps 32 rays (with 2 rays a pixel and 80,000 pixels,
-// 46 us in tiles of 8, 38 in tiles of 16). A tile that the caller chose stays.
-static void small_frame_tiles(const vxl_ctx* ctx, int64_t npix, int R, vxl_tuning& t) {
+// part of the GPU, while large frames want large pools, and pools of fewer
+// rays than a warp has lanes lose more than the shorter chain gives. Each
+// halving is taken where it measured faster (us in tiles of 2, 4, 8, 16 pixels
+// on 512^3 / on a 1024^3 terrain, whose rays are long and differ more):
+//  6 rays a pixel
+//     5,400 pixels    48   53   54   61  /   56   59   66  102
+//    40,000           88   71   65   69  /  102   82   76  115
+//    79,200          146  105   90   77  /  183  122   92  125
+//   120,000          200  137  109   97  /  264  163  115  132
+// 10 rays
+//    14,560           55   55   62   81  /   70   67   91  151
+//    40,000           93   77   70   86  /  107   85  100  162
+//   120,000          212  155  126  131  /  270  176  169  209
+//   256,000          371  258  200  188  /  459  280  233  334
+// 18 rays
+//     5,400           52   59   71  114  /   62   81  132  236
+//    14,560           59   61   77  129  /   73   85  137  243
+//    40,000          106   92   90  142  /  122  103  150  256
+// A tile that the caller chose stays.
+static void small_frame_tiles(const vxl_ctx* ctx, int64_t npix, int R, bool wide, vxl_tuning& t) {
     if (ctx->tile_chosen || t.kstep != 8 || t.grab != 1 || t.tile_w != t.tile_px || t.tile_px > 16) return;
     const int64_t warps = (int64_t)ctx->sm_count * 32;
     while (t.tile_px > 2 && t.tile_px / 2 * R >= 32) {
-        // tiles per warp below which the half is faster: 2.5 for 16, 0.75 for 8, 0.4 for 4
-        const int64_t pct = t.tile_px == 16 ? 250 : (t.tile_px == 8 ? 75 : 40);
+        // tiles per warp below which the half is faster, in hundredths
+        const int64_t pct = t.tile_px == 16 ? (R >= 10 ? 250 : (wide ? 175 : 65)) : (t.tile_px == 8 ? 75 : 40);
         if (npix * 100 >= warps * t.tile_px * pct) break;
         t.tile_px = t.tile_w = t.tile_px / 2;
     }
@@ -1187,7 +1196,7 @@ vxl_status launch_trace_occlusion_lean(vxl_ctx* ctx, const vxl_grid* g, const vx
         t.tile_px = 8;
         t.tile_w = 8;
     }
-    small_frame_tiles(ctx, gb->npix, R, t);
+    small_frame_tiles(ctx, gb->npix, R, g->tl_wide, t);
     if (g->tl_wide) {
         LeanSceneW PW;
         PW.S = scene_of(g, gb, p, out, t);
@@ -1235,7 +1244,7 @@ vxl_tuning lean_batch_tuning(const vxl_ctx* ctx, const vxl_batch_item* items, in
     }
     int64_t npix = 0;
     for (int i = 0; i < n; i++) npix += items[i].gbuf.npix;
-    small_frame_tiles(ctx, npix, mr, t);
+    small_frame_tiles(ctx, npix, mr, false, t);
     return t;
 }
 
