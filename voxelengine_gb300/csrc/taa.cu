@@ -22,6 +22,8 @@
 // 60% issue-bound, the rest load latency.
 // Planes rather than records: the 16-byte loads of scattered taps then spread
 // over eight L1 bank groups (texel mod 8).
+#include <climits>
+
 #include "vxl_device.cuh"
 #include "vxl_internal.h"
 
@@ -39,6 +41,10 @@ struct TaaIn {
     const float* noise;     // 4
     int W, H;
 };
+
+// The pass's launches follow one another with their starts overlapped (taa_launch):
+// this waits for the one before to end and its writes to be seen.
+__device__ __forceinline__ void after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 __device__ __forceinline__ float gmax(float x, float y) { return (x < y) ? y : x; }
 __device__ __forceinline__ float gmin(float x, float y) { return (y < x) ? y : x; }
@@ -178,7 +184,7 @@ __global__ void __launch_bounds__(kPackW* kPackH) k_taa_pack(const TaaIn I, floa
         rec[n + (size_t)(y0 + ly) * I.W + x0 + lx] = make_float4(s_val[0][c], s_val[1][c], s_val[2][c], __int_as_float(f));
     }
     if (t0 == 0) {
-        if (blockIdx.x == 0 && blockIdx.y == 0) list[0] = 0;
+        if (blockIdx.x == 0 && blockIdx.y == 0) list[0] = list[1] = 0;
         for (int w = 1; w < kPackW * kPackH / 32; w++) top = fmaxf(top, s_max[w]);
         motion_max[blockIdx.y * gridDim.x + blockIdx.x] = top;
     }
@@ -294,12 +300,46 @@ __device__ __forceinline__ float4 disocc_tap(const TaaIn& I, const float4* __res
     return make_float4(factor * ld[0], factor * ld[1], factor * ld[2], factor);
 }
 
+// The same with every texel loaded at once: a warp of neighbouring pixels,
+// which together need most of them, waits for memory once a tap.
+__device__ __forceinline__ float4 disocc_tap_all(const TaaIn& I, const float4* __restrict__ rec, float iResx, float iResy,
+                                                 const Centre& c, bool still, int x, int y) {
+    const float FAR = 4096.0f;
+    const float ox = (float)x * iResx, oy = (float)y * iResy;
+    const float u = clampg(c.uvx + ox, 0.001f, 0.999f), v = clampg(c.uvy + oy, 0.001f, 0.999f);
+    const TapAt t(I.W, I.H, u, v);
+    const size_t n = (size_t)I.W * I.H;
+    const float4* mat = reinterpret_cast<const float4*>(I.material);
+    float ld[4], co[4], no[4], ma[4];
+    t.get(mat, __ldg(mat + t.i00), false, ma);
+    t.get(rec + 2 * n, __ldg(rec + 2 * n + t.i00), false, no);
+    t.get(rec + n, __ldg(rec + n + t.i00), false, co);
+    t.get(rec, __ldg(rec + t.i00), false, ld);
+    float factor = gmax(dot3(c.no, no), 0.0f);
+    factor *= glsl_step(0.8f, 1.0f - len4(c.ma, ma));
+    factor *= 1.0f - clampg(fabsf(c.de - ld[3]) * FAR, 0.0f, 1.0f);
+    factor *= 1.0f - clampg(len3(c.co, co), 0.0f, 1.0f);
+    if (!still) {
+        float mo[2];
+        t.motion(I.motion, mo);
+        if (len2(c.mo[0] - mo[0], c.mo[1] - mo[1]) > 0.1f) factor = 0.0f;
+    }
+    return make_float4(factor * ld[0], factor * ld[1], factor * ld[2], factor);
+}
+
 // 1.212 - radius / 12 of the spiral's taps (LightTAA.frag:115)
 __constant__ float c_ring[12] = {1.212f - 2.0f / 12.0f, 1.212f - 3.0f / 12.0f,  1.212f - 4.0f / 12.0f,  1.212f - 5.0f / 12.0f,
                                  1.212f - 6.0f / 12.0f, 1.212f - 7.0f / 12.0f,  1.212f - 8.0f / 12.0f,  1.212f - 9.0f / 12.0f,
                                  1.212f - 10.0f / 12.0f, 1.212f - 11.0f / 12.0f, 1.212f - 12.0f / 12.0f, 1.212f - 13.0f / 12.0f};
 
 constexpr int kDisTaps = 19 * 19;
+
+// The list of disoccluded pixels: how many lie in warps of few and in warps of
+// more than kTaaFew, then the former from the front, the latter from the back.
+constexpr int kTaaFew = 16;
+__device__ __forceinline__ unsigned taa_entry(unsigned n, bool many, int at) {
+    return many ? n + 1u - (unsigned)at : 2u + (unsigned)at;
+}
 
 // The centre of a pixel: everything its taps are compared with; returns its
 // flags. A warp's centres are neighbours, so all four texels are loaded at
@@ -352,24 +392,27 @@ __device__ __forceinline__ bool taa_still(int W, int H, int tx, int ty, const fl
 // pixels, at the screen's edge, ran on after all others (1080p, 1% of the
 // pixels: 958 us, now 456 for the spiral and 126 here).
 // A block of 384 threads makes a pixel's taps in one go, for few pixels; many
-// run better in blocks of 128.
+// run better in blocks of 128. `apart` or more pixels in warps of many are left
+// to k_taa_many.
 constexpr int kEdgeGroup = 4;
 template <int THREADS>
-__global__ void __launch_bounds__(THREADS) k_taa_edge(const TaaIn I, const float4* __restrict__ rec,
+__global__ void __launch_bounds__(THREADS, THREADS == 128 ? 8 : 2) k_taa_edge(const TaaIn I, const float4* __restrict__ rec,
                                                   const float* __restrict__ motion_max, const int* __restrict__ list,
-                                                  float* __restrict__ out) {
+                                                  int apart, float* __restrict__ out) {
     __shared__ float4 s_dis[kEdgeGroup][kDisTaps];
     __shared__ Centre s_centre[kEdgeGroup];
-    __shared__ int s_flags[kEdgeGroup];
+    __shared__ int s_flags[kEdgeGroup], s_pixel[kEdgeGroup];
     __shared__ bool s_still[kEdgeGroup];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const float iResx = 1.0f / (float)I.W, iResy = 1.0f / (float)I.H;
-    const int count = list[0];
+    const unsigned n = (unsigned)I.W * (unsigned)I.H;
+    after_previous();
+    const int few = list[0], many = list[1], count = many >= apart ? few : few + many;
     const int group = min(kEdgeGroup, (count + (int)gridDim.x - 1) / (int)gridDim.x);
     for (int k = blockIdx.x * group; k < count; k += gridDim.x * group) {
         const int m = min(group, count - k);
         if (wib < m) {
-            const int i = list[1 + k + wib];
+            const int e = k + wib, i = list[taa_entry(n, e >= few, e < few ? e : e - few)];
             Centre c;
             const int f = taa_centre(I, rec, i % I.W, i / I.W, c);
             const bool still = taa_still(I.W, I.H, i % I.W / kPackW, i / I.W / kPackH, motion_max);
@@ -377,6 +420,7 @@ __global__ void __launch_bounds__(THREADS) k_taa_edge(const TaaIn I, const float
                 s_still[wib] = still;
                 s_centre[wib] = c;
                 s_flags[wib] = f;
+                s_pixel[wib] = i;
             }
         }
         __syncthreads();
@@ -397,9 +441,78 @@ __global__ void __launch_bounds__(THREADS) k_taa_edge(const TaaIn I, const float
             }
             const float total = __shfl_sync(0xffffffffu, acc, lane | 3);
             if (lane < 4 * m)
-                out[4 * (size_t)list[1 + k + (lane >> 2)] + (lane & 3)] = (lane & 3) < 3 ? acc / total : 1.0f;
+                out[4 * (size_t)s_pixel[lane >> 2] + (lane & 3)] = (lane & 3) < 3 ? acc / total : 1.0f;
         }
         __syncthreads();
+    }
+}
+
+// The pixels in warps of many, one a lane, where there are enough of them to
+// fill the GPU that way (a fast pan, a camera that jumps): a warp's pixels
+// share texels, and all 16 loads of a tap are in flight. That takes 128
+// registers, which is why this is a kernel of its own: with k_taa_edge's 64 it
+// took a third longer, and k_taa_edge 8% longer with 128. us a frame at 1080p
+// for 2, 4, 8, 25 and 100% of the frame's rows, by k_taa_edge / here: 732 /
+// 786, 993 / 1045, 1486 / 1275, 3640 / 2562, 13061 / 8172; at 640x360 for 25,
+// 50 and 100%: 437 / 433, 773 / 665, 1473 / 931. L1 wavefronts bound it (71%).
+constexpr int kTaaMany = 560;  // pixels per SM from which on it runs
+constexpr int kManyThreads = 128;
+__global__ void __launch_bounds__(kManyThreads, 4) k_taa_many(const TaaIn I, const float4* __restrict__ rec,
+                                                              const int* __restrict__ list, int apart,
+                                                              float* __restrict__ out) {
+    after_previous();
+    const int many = list[1], lane = threadIdx.x & 31;
+    if (many >= apart) {
+        const unsigned n = (unsigned)I.W * (unsigned)I.H;
+        const float iResx = 1.0f / (float)I.W, iResy = 1.0f / (float)I.H;
+        for (int k = blockIdx.x * kManyThreads + threadIdx.x - lane; k < many; k += gridDim.x * kManyThreads) {
+            const bool on = k + lane < many;
+            const int i = list[taa_entry(n, true, on ? k + lane : k)], px = i % I.W, py = i / I.W;
+            // The motion test loads nothing where the motions of all texels in
+            // reach (9 pixels and the clamp at 0.001, and one for the second
+            // texel) differ by less than 0.1, rounding included.
+            const int x0 = max(__reduce_min_sync(0xffffffffu, px) - 10, 0), x1 = min(__reduce_max_sync(0xffffffffu, px) + 10, I.W - 1);
+            const int y0 = max(__reduce_min_sync(0xffffffffu, py) - 10, 0), y1 = min(__reduce_max_sync(0xffffffffu, py) + 10, I.H - 1);
+            const int w = x1 - x0 + 1, texels = w * (y1 - y0 + 1);
+            bool still = I.W <= 9000 && I.H <= 9000 && texels <= 4096;
+            if (still) {
+                float lo0 = INFINITY, hi0 = -INFINITY, lo1 = INFINITY, hi1 = -INFINITY;
+                bool ok = true;
+                for (int t = lane; t < texels; t += 32) {
+                    const float2 m = __ldg(reinterpret_cast<const float2*>(I.motion) + (size_t)(y0 + t / w) * I.W + x0 + t % w);
+                    ok = ok && fabsf(m.x) < 256.0f && fabsf(m.y) < 256.0f;
+                    lo0 = fminf(lo0, m.x);
+                    hi0 = fmaxf(hi0, m.x);
+                    lo1 = fminf(lo1, m.y);
+                    hi1 = fmaxf(hi1, m.y);
+                }
+                for (int o = 16; o > 0; o >>= 1) {
+                    lo0 = fminf(lo0, __shfl_xor_sync(0xffffffffu, lo0, o));
+                    hi0 = fmaxf(hi0, __shfl_xor_sync(0xffffffffu, hi0, o));
+                    lo1 = fminf(lo1, __shfl_xor_sync(0xffffffffu, lo1, o));
+                    hi1 = fmaxf(hi1, __shfl_xor_sync(0xffffffffu, hi1, o));
+                }
+                still = __all_sync(0xffffffffu, ok) && hi0 - lo0 < 2.0f * kTaaStill && hi1 - lo1 < 2.0f * kTaaStill;
+            }
+            if (!on) continue;
+            Centre c;
+            taa_centre(I, rec, px, py, c);
+            float4 sum = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            for (int x = -9; x <= 9; x++)
+#pragma unroll 1
+                for (int y = -9; y <= 9; y++) {
+                    const float4 t = disocc_tap_all(I, rec, iResx, iResy, c, still, x, y);
+                    sum.x += t.x;
+                    sum.y += t.y;
+                    sum.z += t.z;
+                    sum.w += t.w;
+                }
+            float* o = out + 4 * (size_t)i;
+            o[0] = sum.x / sum.w;
+            o[1] = sum.y / sum.w;
+            o[2] = sum.z / sum.w;
+            o[3] = 1.0f;
+        }
     }
 }
 
@@ -421,6 +534,7 @@ __global__ void __launch_bounds__(32 * kTaaRows, BLOCKS) k_taa(const TaaIn I, co
     const int i = valid ? py * W + px : 0;
     const size_t n = (size_t)W * H;
     const float4* mat = reinterpret_cast<const float4*>(I.material);
+    after_previous();
     const bool still = taa_still(W, H, (int)(blockIdx.x * WIDE / kPackW), (int)(blockIdx.y * kTaaRows / kPackH), motion_max);
     const float GR = 2.118033988749895f;
     const float iResx = 1.0f / (float)W, iResy = 1.0f / (float)H;
@@ -445,10 +559,11 @@ __global__ void __launch_bounds__(32 * kTaaRows, BLOCKS) k_taa(const TaaIn I, co
     }
     const unsigned dis = __ballot_sync(0xffffffffu, mode == 1 && share == 0);
     if (dis != 0u) {
+        const bool many = __popc(dis) > kTaaFew;
         int at = 0;
-        if (lane == 0) at = atomicAdd(list, __popc(dis));
-        at = __shfl_sync(0xffffffffu, at, 0);
-        if (mode == 1 && share == 0) list[1 + at + __popc(dis & ((1u << lane) - 1u))] = i;
+        if (lane == 0) at = atomicAdd(list + many, __popc(dis));
+        at = __shfl_sync(0xffffffffu, at, 0) + __popc(dis & ((1u << lane) - 1u));
+        if (mode == 1 && share == 0) list[taa_entry((unsigned)n, many, at)] = i;
     }
     if (mode != 2) return;  // with its pixel's other lanes
     const float* motion = c.mo;
@@ -551,6 +666,22 @@ __global__ void __launch_bounds__(32 * kTaaRows, BLOCKS) k_taa(const TaaIn I, co
     o[3] = clampg(lastVariance * 0.7f, 0.0f, 1.0f);
 }
 
+// A launch whose start overlaps the end of the one before it in the stream
+// (after_previous waits in the kernel): 1 to 2 us less between two of them.
+template <class... P, class... A>
+cudaError_t taa_launch(void (*kernel)(P...), dim3 grid, unsigned threads, cudaStream_t s, A... args) {
+    cudaLaunchAttribute overlap[1];
+    overlap[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    overlap[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.stream = s;
+    cfg.attrs = overlap;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, (P)args...);
+}
+
 }  // namespace
 
 vxl_status launch_light_taa(vxl_ctx* ctx, const vxl_taa_frame* f, float* out, cudaStream_t s) {
@@ -558,9 +689,9 @@ vxl_status launch_light_taa(vxl_ctx* ctx, const vxl_taa_frame* f, float* out, cu
             f->height};
     const size_t n = (size_t)f->width * f->height;
     const dim3 pack((unsigned)((f->width + kPackW - 1) / kPackW), (unsigned)((f->height + kPackH - 1) / kPackH));
-    // planes, the pre-pass's maxima, and the list of disoccluded pixels (its length first)
+    // planes, the pre-pass's maxima, and the list of disoccluded pixels (its lengths first)
     const size_t planes = n * kTaaPlanes * sizeof(float4), maxima = (size_t)pack.x * pack.y * sizeof(float);
-    VXL_TRY(ctx_grow(&ctx->d_taa, &ctx->taa_bytes, planes + maxima + (n + 1) * sizeof(int)));
+    VXL_TRY(ctx_grow(&ctx->d_taa, &ctx->taa_bytes, planes + maxima + (n + 2) * sizeof(int)));
     float4* rec = (float4*)ctx->d_taa;
     float* motion_max = (float*)((char*)ctx->d_taa + planes);
     int* list = (int*)((char*)ctx->d_taa + planes + maxima);
@@ -572,19 +703,19 @@ vxl_status launch_light_taa(vxl_ctx* ctx, const vxl_taa_frame* f, float* out, cu
     // runs in larger blocks (us, four lanes a pixel / one: 5,000 pixels 25 / 42,
     // 40,000 38 / 47, 58,000 44 / 49, 80,000 54 / 54, 120,000 66 / 60).
     const bool small = n <= (size_t)ctx->sm_count * 448;
+    const int apart = small ? INT_MAX : ctx->sm_count * kTaaMany;
+    const unsigned edge = (unsigned)std::min<size_t>(n, (size_t)ctx->sm_count * (small ? 2 : 8));
     if (small) {
         const dim3 quarter((unsigned)((f->width + 7) / 8), grid.y);
-        k_taa<4, 7><<<quarter, 32 * kTaaRows, 0, s>>>(I, rec, motion_max, list, out);
+        VXL_TRY_CUDA(taa_launch(k_taa<4, 7>, quarter, 32 * kTaaRows, s, I, rec, motion_max, list, out));
+        VXL_TRY_CUDA(taa_launch(k_taa_edge<384>, edge, 384, s, I, rec, motion_max, list, apart, out));
+        ctx->launches += 2;
     } else {
-        k_taa<1, 7><<<grid, 32 * kTaaRows, 0, s>>>(I, rec, motion_max, list, out);
+        VXL_TRY_CUDA(taa_launch(k_taa<1, 7>, grid, 32 * kTaaRows, s, I, rec, motion_max, list, out));
+        VXL_TRY_CUDA(taa_launch(k_taa_edge<128>, edge, 128, s, I, rec, motion_max, list, apart, out));
+        VXL_TRY_CUDA(taa_launch(k_taa_many, (unsigned)ctx->sm_count * 4, kManyThreads, s, I, rec, list, apart, out));
+        ctx->launches += 3;
     }
-    ctx->launches++;
-    const unsigned edge = (unsigned)std::min<size_t>(n, (size_t)ctx->sm_count * (small ? 2 : 8));
-    if (small)
-        k_taa_edge<384><<<edge, 384, 0, s>>>(I, rec, motion_max, list, out);
-    else
-        k_taa_edge<128><<<edge, 128, 0, s>>>(I, rec, motion_max, list, out);
-    ctx->launches++;
     VXL_TRY_CUDA(cudaGetLastError());
     return VXL_OK;
 }
