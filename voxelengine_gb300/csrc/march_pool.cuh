@@ -134,10 +134,11 @@ __device__ __forceinline__ bool march_outside(const GridView& g, f3 p, f3 e) {
 // The N tests from p on, s apart: bit j of the result set where test j finds a
 // voxel. q becomes the position after them. `in`: p is known to lie in [0, n)
 // (it becomes so for q's batch); skip: that nothing can be hit; small:
-// march_small(s); left: nothing can be hit from q on.
-template <bool FINE, int N>
-__device__ __forceinline__ unsigned march_tests(const GridView& g, f3 p, f3 s, f3& q, bool& in, bool skip, bool small,
-                                                bool& left) {
+// march_small(s); left: nothing can be hit from q on. lanes: those that call it
+// together, from a vote of the whole warp.
+template <bool FINE, int N, int EDGE>
+__device__ __forceinline__ unsigned march_tests(unsigned lanes, const GridView& g, f3 p, f3 s, f3& q, bool& in, bool skip,
+                                                bool small, bool& left) {
     // where the last test lies, to far less than the half cell that the bounds leave
     const f3 e = mk(__fmaf_rn(s.x, (float)(N - 1), p.x), __fmaf_rn(s.y, (float)(N - 1), p.y),
                     __fmaf_rn(s.z, (float)(N - 1), p.z));
@@ -149,7 +150,7 @@ __device__ __forceinline__ unsigned march_tests(const GridView& g, f3 p, f3 s, f
     const bool none = !inner && (skip || (small && march_outside(g, p, e)));
     // One lane on the grid's edge sends its whole warp through the tests that
     // look at every position: a branch per lane would run both loops.
-    if (__all_sync(__activemask(), inner || none)) {
+    if (__all_sync(lanes, inner || none)) {
         if (inner) {
 #pragma unroll
             for (int j = 0; j < N; j++) {
@@ -161,7 +162,7 @@ __device__ __forceinline__ unsigned march_tests(const GridView& g, f3 p, f3 s, f
             left = march_gone(g, q, s);
         }
     } else {
-#pragma unroll 1
+#pragma unroll EDGE
         for (int j = 0; j < N; j++) {
             hits |= march_bit<FINE>(g, q, !none && march_inside(g, q)) ? 1u << j : 0u;
             q = add(q, s);
@@ -183,7 +184,7 @@ __device__ __forceinline__ float march_dcoarse(uint32_t id) { return (id & kMarc
 // part, which are the pool's first ones then. Rays that ended wait until no
 // more than kMarchRefill lanes run: their ends and the refill cost about as
 // much as a batch of tests.
-template <bool FINE, bool REC, class Done>
+template <bool FINE, bool REC, int EDGE, class Done>
 __device__ __forceinline__ int march_part(const GridView& g, MarchPool& P, int count, Done done) {
     constexpr int N = kMarchBatch;
     int base = 0, kept = 0;
@@ -216,7 +217,7 @@ __device__ __forceinline__ int march_part(const GridView& g, MarchPool& P, int c
         }
         const int waiting = base < count ? kMarchRefill : 0;
         bool run = busy, left = false;
-        unsigned hits = 0u;
+        unsigned hits = 0u, lanes = __ballot_sync(0xffffffffu, run);
         do {
             if (REC && run && ghost) {
                 // out of the grid for good: on to the last tests without looking
@@ -227,7 +228,7 @@ __device__ __forceinline__ int march_part(const GridView& g, MarchPool& P, int c
             }
             if (run) {
                 f3 q;
-                hits = march_tests<FINE, N>(g, p, s, q, in, REC && ghost, small, left);
+                hits = march_tests<FINE, N, EDGE>(lanes, g, p, s, q, in, REC && ghost, small, left);
                 const float dn = d + (float)N * ds;  // small multiples of 0.5: exact
                 if (hits != 0u || !(dn < lim) || (left && !REC)) {
                     run = false;
@@ -237,7 +238,8 @@ __device__ __forceinline__ int march_part(const GridView& g, MarchPool& P, int c
                     ghost = REC && (ghost || left);
                 }
             }
-        } while (__popc(__ballot_sync(0xffffffffu, run)) > waiting);
+            lanes = __ballot_sync(0xffffffffu, run);
+        } while (__popc(lanes) > waiting);
         bool keep = false;
         if (busy && !run) {
             int nv = 1;  // the batch's tests that the shader makes: those at a distance below lim
@@ -277,17 +279,17 @@ __device__ __forceinline__ int march_part(const GridView& g, MarchPool& P, int c
 
 // Both parts. The warp has written the pool's rays; those whose origin or
 // direction is outside ray_domain_ok are left out by the caller (misses).
-template <bool REC, class Done>
+template <bool REC, int EDGE = 1, class Done>
 __device__ __forceinline__ void march_pool(const GridView& g, MarchPool& P, int count, Done done) {
     __syncwarp();
-    const int kept = march_part<true, REC>(g, P, count, done);
-    march_part<false, REC>(g, P, kept, done);
+    const int kept = march_part<true, REC, EDGE>(g, P, count, done);
+    march_part<false, REC, EDGE>(g, P, kept, done);
 }
 
 // The first kMarchFirst tests of one ray per lane with `on` set (a quarter of
 // the rays or more end there, and neighbours' first tests run alike), then
 // the ray into the pool unless it has ended.
-template <bool REC, class Done>
+template <bool REC, int EDGE = 1, class Done>
 __device__ __forceinline__ void march_push(const GridView& g, MarchPool& P, int& count, bool on, f3 o, f3 d,
                                            float dist, uint32_t id, Done done) {
     static_assert(kMarchFirst < 6, "the SuperSparse marcher's fine part is 6 tests");
@@ -295,9 +297,10 @@ __device__ __forceinline__ void march_push(const GridView& g, MarchPool& P, int&
     const float step0 = march_step0(id);
     const f3 s = mul(d, step0);
     f3 q = o;
+    const unsigned lanes = __ballot_sync(0xffffffffu, on);
     if (on) {
         bool in = o.x >= 0.0f && o.y >= 0.0f && o.z >= 0.0f && march_inside(g, o), left = false;
-        const unsigned hits = march_tests<true, kMarchFirst>(g, o, s, q, in, false, march_small(s), left);
+        const unsigned hits = march_tests<true, kMarchFirst, EDGE>(lanes, g, o, s, q, in, false, march_small(s), left);
         if (hits) {
             const int k = __ffs(hits) - 1;
             f3 p = o;

@@ -421,9 +421,10 @@ __device__ __forceinline__ void lean_tile(const SceneDesc& S, const LeanGrid& L,
         bool run = busy;
         int end = 0;  // 1 set cell, 2 miss, 3 hit at ht
         float ht = 0.0f;
+        unsigned running = __ballot_sync(0xffffffffu, run);
         do {
             if (run) {
-                if (__all_sync(__activemask(), n + KSTEP <= 256)) {
+                if (__all_sync(running, n + KSTEP <= 256)) {
                     end = lean_batch<KSTEP>(L.w, ax, ay, az, tx, ty, tz, tdx, tdy, tdz, kx, ky, kz,
                                                       keep_y, keep_z, one, two27, maxt, tot);
                     if (end == 0) {
@@ -451,7 +452,8 @@ __device__ __forceinline__ void lean_tile(const SceneDesc& S, const LeanGrid& L,
                 }
                 run = end == 0;
             }
-        } while (__popc(__ballot_sync(0xffffffffu, run)) > waiting);
+            running = __ballot_sync(0xffffffffu, run);
+        } while (__popc(running) > waiting);
         if (busy && !run) {
             if (end == 3 || (end == 1 && lean_set_cell(L, ax, ay, az, tx, ty, tz, tot, maxt, &ht))) {
                 const int k = (meta >> 9) & 31, pp = (meta >> 4) & 31;

@@ -283,9 +283,9 @@ __global__ void __launch_bounds__(1024) k_soft_bwd(const SoftConsts c, const flo
                                                    const float* __restrict__ light, float4* __restrict__ grad) {
     const int lane = threadIdx.x & 31, k = threadIdx.x >> 5;
     const int pix = blockIdx.x * 32 + lane;
-    if (pix >= c.npix) return;
     f3 O, D;
-    const int s = pixel_setup(c, pix, k, &O, &D);
+    const int s = pix < c.npix ? pixel_setup(c, pix, k, &O, &D) : -1;
+    const unsigned lanes = __ballot_sync(0xffffffffu, s >= 0);
     if (s < 0) return;
     const float g0 = gimg[3 * pix], g1 = gimg[3 * pix + 1], g2 = gimg[3 * pix + 2];
     const float4 rs = __ldg(c.vox + s);
@@ -319,7 +319,7 @@ __global__ void __launch_bounds__(1024) k_soft_bwd(const SoftConsts c, const flo
     // end: entries of one position lie side by side in local memory (each lane
     // from its own end read four times the sectors, most of them past L1:
     // 786 us against 698, and 879 before the batched walk).
-    const int longest = __reduce_max_sync(__activemask(), m);
+    const int longest = __reduce_max_sync(lanes, m);
     for (int j0 = (longest - 1) / kSoftBatch * kSoftBatch; j0 >= 0; j0 -= kSoftBatch) {
         int2 ce[kSoftBatch];
         float4 vs[kSoftBatch];

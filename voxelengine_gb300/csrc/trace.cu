@@ -99,9 +99,10 @@ __global__ void __launch_bounds__(32 * kMarchWarps, kMarchBlocks)
         } else if (idle == 0xffffffffu && next >= n) {
             break;
         }
+        const unsigned running = __ballot_sync(0xffffffffu, busy);
         if (busy) {
             Hit h;
-            if (dda_run<false, CACHE, !CACHE, true>(g, s, h, kRayBatch)) {
+            if (dda_run<false, CACHE, !CACHE, true>(g, s, h, kRayBatch, running)) {
                 store_record(rec + id, h);
                 busy = false;
             }

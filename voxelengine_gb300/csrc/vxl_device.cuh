@@ -499,15 +499,16 @@ __device__ __forceinline__ int dda_steps_clear(const GridView& g, DState& s, Hit
 // otherwise it keeps both at every iteration (a per-lane choice would run both
 // loops one after the other). Faster in the single-scene pool, slower in the
 // batched kernel (-10%), which keeps the tests.
+// lanes: those that call this together (SKIP_BOUNDS), best from a vote of the whole warp.
 template <bool LEAP = false, bool CACHE = true, bool ONE_COUNT = false, bool SKIP_BOUNDS = false>
-__device__ __forceinline__ int dda_run(const GridView& g, DState& s, Hit& r, int budget) {
+__device__ __forceinline__ int dda_run(const GridView& g, DState& s, Hit& r, int budget, unsigned lanes = __activemask()) {
     if (SKIP_BOUNDS && !LEAP) {
         const int mx = s.sx > 0 ? (int)g.ux - s.cx : s.cx;
         const int my = s.sy > 0 ? (int)g.uy - s.cy : s.cy;
         const int mz = s.sz > 0 ? (int)g.uz - s.cz : s.cz;
         const bool inside = (unsigned)s.cx <= g.ux && (unsigned)s.cy <= g.uy && (unsigned)s.cz <= g.uz;
         const bool clear = inside && min(min(mx, my), mz) >= budget - 1 && s.n + budget < 256;
-        if (__all_sync(__activemask(), clear)) return dda_steps_clear<CACHE>(g, s, r, budget);
+        if (__all_sync(lanes, clear)) return dda_steps_clear<CACHE>(g, s, r, budget);
     }
     return dda_steps<LEAP, CACHE, ONE_COUNT>(g, s, r, budget);
 }
