@@ -71,3 +71,29 @@ def test_long_reflections(vxl, ctx):
     torch.cuda.synchronize()
     assert 0.1 < (want != 256.0).mean() < 1.0
     assert np.array_equal(out.cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("mode", [1, 2])
+def test_along_the_faces(vxl, ctx, mode):
+    """Rays within half a cell of the faces of a long grid, where positions are rounded most, along them and across."""
+    import torch
+
+    dims, rng, n = (32000, 34, 30), np.random.default_rng(9 + mode), 20000
+    g = np.zeros((15, 17, 16000), np.uint8)
+    for at in (slice(0, 200), slice(15800, 16000)):
+        g[:, :, at] = rng.choice(np.array([0, 0, 0, 0, 0, 0, 0, 1, 64, 255], np.uint8), (15, 17, 200))
+    off = rng.choice([0.0, 1.0 / 64, 1.0 / 32, 3.0 / 64, 0.2, 0.4999, 0.5, -1.0 / 64, -0.3], (n, 3))
+    o = np.where(rng.random((n, 3)) < 0.5, off, np.array(dims) - off)
+    inner = rng.random((n, 3)) < 0.5
+    o[inner] = (rng.random((n, 3)) * dims)[inner]
+    o[:, 0] = np.where(rng.random(n) < 0.5, np.minimum(o[:, 0], 390.0), np.maximum(o[:, 0], 31610.0))
+    d = rng.normal(size=(n, 3)) * rng.choice([0.0, 1.0, 1.0, 1e-3], (n, 3))
+    d[np.abs(d).max(1) == 0.0] = [1.0, 0.0, 0.0]
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    rays = np.concatenate([o, d, rng.choice([128.0, 256.0, 40.0], (n, 1))], 1).astype(F)
+    rec = rec_buffer(n)
+    vxl.trace_rays(ctx, grid_from_r8(vxl, ctx, g), dev(rays), n, mode, rec)
+    torch.cuda.synchronize()
+    want = oracle.trace_rays(g, rays, mode=mode)
+    assert 0.1 < (want["flags"] & 1).mean() < 1.0
+    assert_recs_equal(recs_np(rec), want)
