@@ -1,11 +1,16 @@
 // The voxelizer's host side (csrc/vxl_api.cpp) on a CUDA runtime of this file's
-// own: copies wait in a queue until something synchronises, as a GPU's do, and
-// the n-th call after the tables' upload fails. Prints, per n, the status of
-// the call and how many copies its return left waiting.
+// own: copies wait in a queue until something synchronises, as a GPU's do.
+// Without arguments the n-th call after the tables' upload fails; prints, per
+// n, the status of the call and how many copies its return left waiting. With
+// the name of a list and its length: orders that list, checks the order, and
+// prints its levels and the fastest of three calls in ms.
+#include <chrono>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
 #include <functional>
+#include <random>
+#include <string>
 #include <vector>
 
 #include "vxl_internal.h"
@@ -58,16 +63,73 @@ void trace_layout_dims(vxl_grid* g) { g->tl_nwords = 0; }
 vxl_status launch_build_tile_mask(vxl_grid*, cudaStream_t) {
     return failing() ? fail(VXL_ERR_CUDA, "tile mask") : VXL_OK;
 }
-vxl_status launch_voxelize_level(vxl_grid*, const VoxJob*, const uint64_t*, const DevModel*, int, int, uint64_t,
-                                 int32_t*, cudaStream_t) {
+static std::vector<int> levels_;  // first job of each level launched
+static const VoxJob* jobs_;
+vxl_status launch_voxelize_level(vxl_grid*, const VoxJob* jobs, const uint64_t*, const DevModel*, int job0, int,
+                                 uint64_t, int32_t*, cudaStream_t) {
+    levels_.push_back(job0);
+    jobs_ = jobs;
     return failing() ? fail(VXL_ERR_CUDA, "level") : VXL_OK;
 }
 }  // namespace vxl
 
-int main() {
+// Cells of a model of one voxel by axis-aligned placements: bounds of the image in the reference's arithmetic.
+static void cells(const float* m, const vxl_model& M, int* lo, int* hi) {
+    const int last[3] = {M.sx - 1, M.sy - 1, M.sz - 1};
+    for (int a = 0; a < 3; a++) {
+        lo[a] = (int)(m[12 + a] * 10.0f);
+        hi[a] = (int)((m[12 + a] + m[5 * a] * 0.1f * (float)last[a]) * 10.0f);
+    }
+}
+
+static int order(vxl_ctx* ctx, vxl_grid* grid, const std::string& list, int n) {
+    static const uint8_t voxels[64] = {};
+    const vxl_model model{voxels, 4, 4, 4};
+    std::mt19937 rng(n);
+    std::uniform_real_distribution<float> at(0.2f, 2.6f);
+    std::vector<vxl_instance> inst((size_t)n);
+    for (int i = 0; i < n; i++) {
+        vxl_instance& I = inst[(size_t)i];
+        std::memset(&I, 0, sizeof I);
+        I.matrix[0] = I.matrix[5] = I.matrix[10] = I.matrix[15] = 1.0f;
+        for (int a = 0; a < 3; a++) I.matrix[12 + a] = at(rng);
+        I.op = list == "one" ? (i != n / 2) : list == "halves" ? (i >= n / 2) : list == "pairs" ? i % 2 : rng() % 3 != 0;
+    }
+    double best = 1e9;
+    for (int rep = 0; rep < 3; rep++) {
+        vxl::levels_.clear();
+        const auto t = std::chrono::steady_clock::now();
+        if (vxl_voxelize(ctx, grid, &model, 1, inst.data(), n, nullptr, nullptr)) return 2;
+        best = std::min(best, std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t).count());
+    }
+    // every instance once, and after the earlier ones of the other op that share cells with it
+    std::vector<int> level((size_t)n, -1);
+    for (size_t l = 0; l < vxl::levels_.size(); l++)
+        for (int k = vxl::levels_[l]; k < (l + 1 < vxl::levels_.size() ? vxl::levels_[l + 1] : n); k++) {
+            const vxl::VoxJob& J = vxl::jobs_[k];
+            if (J.index < 0 || J.index >= n || level[(size_t)J.index] >= 0) return 3;
+            if (J.op != inst[(size_t)J.index].op || std::memcmp(J.m, inst[(size_t)J.index].matrix, sizeof J.m)) return 4;
+            level[(size_t)J.index] = (int)l;
+        }
+    for (int i = 0; i < n; i++)
+        for (int j = i > 3000 ? i - 3000 : 0; j < i; j++) {
+            if (inst[(size_t)i].op == inst[(size_t)j].op || level[(size_t)j] < level[(size_t)i]) continue;
+            int a[6], b[6];
+            cells(inst[(size_t)i].matrix, model, a, a + 3);
+            cells(inst[(size_t)j].matrix, model, b, b + 3);
+            bool meet = true;
+            for (int k = 0; k < 3; k++) meet = meet && std::max(a[k], b[k]) <= std::min(a[3 + k], b[3 + k]);
+            if (meet) return 5;
+        }
+    std::printf("%zu %.3f\n", vxl::levels_.size(), best);
+    return 0;
+}
+
+int main(int argc, char** argv) {
     vxl_ctx* ctx = nullptr;
     vxl_grid* grid = nullptr;
     if (vxl_ctx_create(0, &ctx) || vxl_grid_create(ctx, 32, 32, 32, &grid)) return 1;
+    if (argc > 2) return order(ctx, grid, argv[1], std::atoi(argv[2]));
     const uint8_t voxel = 20;
     const vxl_model model{&voxel, 1, 1, 1};
     float m[16] = {1, 0, 0, 0, 0, 1, 0, 0, 0, 0, 1, 0, 0.5f, 0.5f, 0.5f, 1};
