@@ -112,7 +112,7 @@ __device__ __forceinline__ void voxel_tile(const GridView& g, unsigned long long
     const uint32_t wxy = wx * wy;
     // the whole image lies inside the grid (the usual tile): its voxels need no
     // bounds, and z is counted up as a float, which holds whole numbers to 2^24
-    const bool inside = gather && z1 <= 1 << 24 && !(__ballot_sync(0xffffffffu, clipped) & 63u);
+    const bool inside = gather && M.sz <= 1 << 24 && !(__ballot_sync(0xffffffffu, clipped) & 63u);
 
     // o = M[3], dx,dy,dz = M[0..2] * 0.1f; wp = o + x*dx + y*dy + z*dz; fwp = ivec3(wp * 10) (:137-147)
     const f3 dz = mk(m[8] * 0.1f, m[9] * 0.1f, m[10] * 0.1f);
@@ -174,10 +174,10 @@ __device__ __forceinline__ void voxel_tile(const GridView& g, unsigned long long
 #pragma unroll
         for (int a = 0; a < 3; a++) {
             const int l = __reduce_min_sync(0xffffffffu, lo[a]), h = __reduce_max_sync(0xffffffffu, hi[a]);
-            // a cell can be INT_MAX or INT_MIN itself (conversions saturate), so each bound is its own test
-            if ((t & 31) == 0) {
-                if (l != INT_MAX) atomicMin(&sh.lo[a], l);
-                if (h != INT_MIN) atomicMax(&sh.hi[a], h);
+            // l > h: no voxel. (Not l == INT_MAX, which a far cell is, too: conversions saturate.)
+            if ((t & 31) == 0 && l <= h) {
+                atomicMin(&sh.lo[a], l);
+                atomicMax(&sh.hi[a], h);
             }
         }
     }
@@ -199,9 +199,9 @@ __device__ __forceinline__ void voxel_tile(const GridView& g, unsigned long long
                 atomicAnd(w, ~b);
         }
     }
-    if (aabb && threadIdx.x < 3) {
-        if (sh.lo[threadIdx.x] != INT_MAX) atomicMin(aabb + threadIdx.x, sh.lo[threadIdx.x]);
-        if (sh.hi[threadIdx.x] != INT_MIN) atomicMax(aabb + 3 + threadIdx.x, sh.hi[threadIdx.x]);
+    if (aabb && threadIdx.x < 3 && sh.lo[threadIdx.x] <= sh.hi[threadIdx.x]) {
+        atomicMin(aabb + threadIdx.x, sh.lo[threadIdx.x]);
+        atomicMax(aabb + 3 + threadIdx.x, sh.hi[threadIdx.x]);
         sh.lo[threadIdx.x] = INT_MAX;
         sh.hi[threadIdx.x] = INT_MIN;
     }
