@@ -227,9 +227,12 @@ __device__ __forceinline__ int lean_batch(const uint32_t* __restrict__ w, uint32
 
 // The batched kernel's warps refill their lanes when no more than this many
 // run (DEFER): the ends of rays and the refill cost about as much as a batch,
-// and taking them together is 1.8% faster on a mix of 24 scenes (500.8 ->
-// 491.8 us; 24 and 28: 0.5% less). The single-scene kernel loses 0.2% at
-// 1080p on 512^3 with it and the wide layout 0.6%: they refill after every batch.
+// and taking them together is 2% faster (2, 24 and 100 scenes of 153,600
+// pixels: 103 -> 101, 1374 -> 1345, 6719 -> 6601 us, runs within 0.5%; 24 and
+// 28: 0.5% less). The single-scene kernel loses 0.2% at 1080p on 512^3 with it
+// and the wide layout 0.6%: they refill after every batch. In a loop of their
+// own: the same loop for both costs the single-scene kernel 1.5% (1045 -> 1061
+// us at 1080p on 512^3).
 constexpr int kLeanRefill = 26;
 
 #ifndef VXL_LEAN_MIN_BLOCKS
@@ -1315,10 +1318,14 @@ static vxl_status launch_lean_batch_k(vxl_ctx* ctx, const LeanScene* d_table, co
         static thread_local LeanBatchParams T;
         std::memset(&T, 0, sizeof(T));
         std::memcpy(T.s, h_table, (size_t)n * sizeof(LeanScene));
-        if (t.kstep <= 4) return launch_lean_batch_pt<TP, 4>(ctx, T, n, max_r, total_tiles, counter, t.grab, s);
+        if constexpr (TP > 4) {  // smaller tiles are chosen with 8 iterations only (small_frame_tiles)
+            if (t.kstep <= 4) return launch_lean_batch_pt<TP, 4>(ctx, T, n, max_r, total_tiles, counter, t.grab, s);
+        }
         return launch_lean_batch_pt<TP, 8>(ctx, T, n, max_r, total_tiles, counter, t.grab, s);
     }
-    if (t.kstep <= 4) return launch_lean_batch_t<TP, 4>(ctx, d_table, n, max_r, total_tiles, counter, t.grab, s);
+    if constexpr (TP > 4) {
+        if (t.kstep <= 4) return launch_lean_batch_t<TP, 4>(ctx, d_table, n, max_r, total_tiles, counter, t.grab, s);
+    }
     return launch_lean_batch_t<TP, 8>(ctx, d_table, n, max_r, total_tiles, counter, t.grab, s);
 }
 
