@@ -18,8 +18,8 @@
 //    (flagged too: 0 times that is not 0);
 //  - the motion test (> 0.1 apart, :120) needs no loads where the pre-pass's
 //    per-tile maxima show that no tap in reach can fail it.
-// 1080p: 1171 + 37 us (every tap 16 16-byte loads) -> 456 + 126 + 41 us, about
-// 60% issue-bound, the rest load latency.
+// 1080p: 1171 + 37 us (every tap 16 16-byte loads) -> 456 + 126 + 41 us, 68%
+// issue-bound, the rest load latency.
 // Planes rather than records: the 16-byte loads of scattered taps then spread
 // over eight L1 bank groups (texel mod 8).
 #include <climits>
@@ -471,15 +471,18 @@ __global__ void __launch_bounds__(kManyThreads, 4) k_taa_many(const TaaIn I, con
             // The motion test loads nothing where the motions of all texels in
             // reach (9 pixels and the clamp at 0.001, and one for the second
             // texel) differ by less than 0.1, rounding included.
-            const int x0 = max(__reduce_min_sync(0xffffffffu, px) - 10, 0), x1 = min(__reduce_max_sync(0xffffffffu, px) + 10, I.W - 1);
-            const int y0 = max(__reduce_min_sync(0xffffffffu, py) - 10, 0), y1 = min(__reduce_max_sync(0xffffffffu, py) + 10, I.H - 1);
+            const int x0 = max(__reduce_min_sync(0xffffffffu, px) - 10, 0);
+            const int x1 = min(__reduce_max_sync(0xffffffffu, px) + 10, I.W - 1);
+            const int y0 = max(__reduce_min_sync(0xffffffffu, py) - 10, 0);
+            const int y1 = min(__reduce_max_sync(0xffffffffu, py) + 10, I.H - 1);
             const int w = x1 - x0 + 1, texels = w * (y1 - y0 + 1);
             bool still = I.W <= 9000 && I.H <= 9000 && texels <= 4096;
             if (still) {
                 float lo0 = INFINITY, hi0 = -INFINITY, lo1 = INFINITY, hi1 = -INFINITY;
                 bool ok = true;
                 for (int t = lane; t < texels; t += 32) {
-                    const float2 m = __ldg(reinterpret_cast<const float2*>(I.motion) + (size_t)(y0 + t / w) * I.W + x0 + t % w);
+                    const size_t at = (size_t)(y0 + t / w) * I.W + x0 + t % w;
+                    const float2 m = __ldg(reinterpret_cast<const float2*>(I.motion) + at);
                     ok = ok && fabsf(m.x) < 256.0f && fabsf(m.y) < 256.0f;
                     lo0 = fminf(lo0, m.x);
                     hi0 = fmaxf(hi0, m.x);

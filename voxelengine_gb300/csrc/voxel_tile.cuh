@@ -8,8 +8,9 @@
 // applies each non-empty word with one 64-bit atomic. A tile's voxels are
 // neighbours, so about 400 of them (the usual 40% fill) land in 50 to 150
 // bricks. One atomic per voxel bound the earlier form: two thousand models
-// (95 M source voxels, 38 M of them set) took 1780 us, now 575 us (640 with one tile shape, bounds tests on every voxel
-// and divisions for every tile's and brick's place).
+// (95 M source voxels, 38 M of them set) took 1780 us, now 575 us (640 with
+// one tile shape, bounds tests on every voxel and divisions for every tile's
+// and brick's place).
 #pragma once
 #include <climits>
 
@@ -142,33 +143,33 @@ __device__ __forceinline__ void voxel_tile(const GridView& g, unsigned long long
         }
     } else {
 #pragma unroll
-    for (int j = 0; j < kVoxPer; j++) {
-        if (pal[j] < 16) continue;
-        const f3 wp = add(oxy, mul(dz, (float)(zf + j * zs)));
-        const int fx = (int)(wp.x * 10.0f), fy = (int)(wp.y * 10.0f), fz = (int)(wp.z * 10.0f);
-        if (aabb) {
-            lo[0] = min(lo[0], fx);
-            lo[1] = min(lo[1], fy);
-            lo[2] = min(lo[2], fz);
-            hi[0] = max(hi[0], fx);
-            hi[1] = max(hi[1], fy);
-            hi[2] = max(hi[2], fz);
+        for (int j = 0; j < kVoxPer; j++) {
+            if (pal[j] < 16) continue;
+            const f3 wp = add(oxy, mul(dz, (float)(zf + j * zs)));
+            const int fx = (int)(wp.x * 10.0f), fy = (int)(wp.y * 10.0f), fz = (int)(wp.z * 10.0f);
+            if (aabb) {
+                lo[0] = min(lo[0], fx);
+                lo[1] = min(lo[1], fy);
+                lo[2] = min(lo[2], fz);
+                hi[0] = max(hi[0], fx);
+                hi[1] = max(hi[1], fy);
+                hi[2] = max(hi[2], fz);
+            }
+            const uint32_t b = bit_index(fx, fy, fz);
+            if (gather && fx >= lx && fx <= hx && fy >= ly && fy <= hy && fz >= lz && fz <= hz) {
+                const uint32_t i = (uint32_t)((fx >> 2) - (lx >> 2)) + (uint32_t)((fy >> 2) - (ly >> 2)) * wx +
+                                   (uint32_t)((fz >> 2) - (lz >> 2)) * wxy;
+                atomicOr(reinterpret_cast<uint32_t*>(sh.bits) + 2u * i + (b >> 5), 1u << (b & 31u));
+            } else if ((unsigned)fx < (unsigned)g.nx && (unsigned)fy < (unsigned)g.ny && (unsigned)fz < (unsigned)g.nz) {
+                // SetVolumeAt bounds: 0 <= x < 2*SizeX (:83). Without a gathered
+                // image, or outside it (a placement that is not finite)
+                unsigned long long* w = words + word_index(g, fx, fy, fz);
+                if (set)
+                    atomicOr(w, 1ull << b);
+                else
+                    atomicAnd(w, ~(1ull << b));
+            }
         }
-        const uint32_t b = bit_index(fx, fy, fz);
-        if (gather && fx >= lx && fx <= hx && fy >= ly && fy <= hy && fz >= lz && fz <= hz) {
-            const uint32_t i = (uint32_t)((fx >> 2) - (lx >> 2)) + (uint32_t)((fy >> 2) - (ly >> 2)) * wx +
-                               (uint32_t)((fz >> 2) - (lz >> 2)) * wxy;
-            atomicOr(reinterpret_cast<uint32_t*>(sh.bits) + 2u * i + (b >> 5), 1u << (b & 31u));
-        } else if ((unsigned)fx < (unsigned)g.nx && (unsigned)fy < (unsigned)g.ny && (unsigned)fz < (unsigned)g.nz) {
-            // SetVolumeAt bounds: 0 <= x < 2*SizeX (:83). Without a gathered
-            // image, or outside it (a placement that is not finite)
-            unsigned long long* w = words + word_index(g, fx, fy, fz);
-            if (set)
-                atomicOr(w, 1ull << b);
-            else
-                atomicAnd(w, ~(1ull << b));
-        }
-    }
     }
     if (aabb) {
 #pragma unroll

@@ -46,8 +46,8 @@ __global__ void __launch_bounds__(kVoxThreads, 12) k_voxelize(GridView g, unsign
 vxl_status launch_voxelize_level(vxl_grid* g, const VoxJob* d_jobs, const uint64_t* d_first, const DevModel* d_models,
                                  int job0, int job1, uint64_t ntiles, int32_t* d_aabb, cudaStream_t s) {
     if (ntiles == 0) return VXL_OK;
-    // 12 blocks of 4 warps fill an SM (42 registers a thread); runs of several
-    // tiles per block spare the searches
+    // 12 blocks of 4 warps are what an SM's registers hold (40 a thread: 48 of
+    // its 64 warps); runs of several tiles per block spare the searches
     const unsigned blocks = (unsigned)std::min<uint64_t>(ntiles, (uint64_t)g->ctx->sm_count * 12);
     k_voxelize<<<blocks, kVoxThreads, 0, s>>>(view_of(g), (unsigned long long*)g->words, d_jobs, d_first, d_models, job0,
                                               job1, d_aabb);
