@@ -97,3 +97,33 @@ def test_along_the_faces(vxl, ctx, mode):
     want = oracle.trace_rays(g, rays, mode=mode)
     assert 0.1 < (want["flags"] & 1).mean() < 1.0
     assert_recs_equal(recs_np(rec), want)
+
+
+@pytest.mark.parametrize("dims", [(6, 10, 14), (40, 34, 52)])
+@pytest.mark.parametrize("n", [1, 33, 129, 20000])
+def test_records_of_rays_that_leave(vxl, ctx, dims, n):
+    """Small grids, which rays leave in their fine part or their coarse one, before their first test or at their last:
+    sparse rays of every length and the light passes' records, which name the last position all the same."""
+    import torch
+
+    rng = np.random.default_rng(n + dims[0])
+    g = oracle.fine_to_r8(rng.random(dims[::-1]) < 0.01)
+    G = grid_from_r8(vxl, ctx, g)
+    o = rng.uniform(-8.0, np.array(dims) + 8.0, (n, 3))
+    d = rng.normal(size=(n, 3)) * rng.choice([0.0, 1.0, 1.0, 4.0], (n, 3))
+    dist = rng.choice([128.0, 256.0, 0.0, -1.0, 15.75, 16.0, 16.5, 17.0, 17.5, 18.0, 20.0, 22.5, 163.0, 164.0, np.inf], (n, 1))
+    rays = np.concatenate([o, d, dist], 1).astype(F)
+    rec = rec_buffer(n)
+    vxl.trace_rays(ctx, G, dev(rays), n, 1, rec)
+    torch.cuda.synchronize()
+    assert_recs_equal(recs_np(rec), oracle.trace_rays(g, rays, mode=1))
+    wcp, nrm = o.astype(F), np.eye(3, dtype=F)[rng.integers(0, 3, n)]
+    depth, noise = rng.uniform(0, 0.3, n).astype(F), rng.random((n, 4)).astype(F)
+    rough, vr = rng.uniform(0.05, 1, n).astype(F), rng.normal(size=(n, 3)).astype(F)
+    rec2, rec1 = rec_buffer(2 * n), rec_buffer(n)
+    a, b, c = (empty(n, torch.float32) for _ in range(3))
+    vxl.light_ambient(ctx, G, dev(wcp), dev(nrm), dev(depth), dev(noise), n, a, b, rec2)
+    vxl.light_reflection(ctx, G, dev(wcp), dev(nrm), dev(vr), dev(rough), dev(noise), n, c, rec1)
+    torch.cuda.synchronize()
+    assert_recs_equal(recs_np(rec2), oracle.light_ambient(g, wcp, nrm, depth, noise)[2].reshape(-1))
+    assert_recs_equal(recs_np(rec1), oracle.light_reflection(g, wcp, nrm, vr, rough, noise)[1].reshape(-1))

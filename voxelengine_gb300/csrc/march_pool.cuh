@@ -18,12 +18,16 @@
 //    the FMA pipe (in shifts and masks, on the ALU pipe: 2 to 6% slower);
 //  - positions are monotone, so one bounds test covers the four steps of a
 //    batch, and a ray outside the grid on the side it moves to is a miss at
-//    once (with records, its positions still advance to the last one).
+//    once; with records its positions still advance to the last one, after the
+//    other rays' tests, 32 such rays side by side (march_away).
 // Before -> after, at 1080p on a 512^3 grid: sun shadow + ambient 391 -> 226
 // us, reflection 364 -> 186 us, the pairs of 64 lights 287 -> 181 us; 1 M
 // incoherent sparse rays with records 271 -> 157 us. Still bound by the
 // instructions it issues (a fine test is about 37, a coarse one 22).
 #pragma once
+#include <cstdint>
+#include <type_traits>
+
 #include "vxl_device.cuh"
 
 namespace vxl {
@@ -39,8 +43,14 @@ struct MarchPool {
     float4 a[kMarchRays];  // position, dist
     float4 b[kMarchRays];  // step, id
 };
-// id: the ray's index in the tile; kMarchSuper set for the SuperSparse marcher
-constexpr uint32_t kMarchSuper = 0x80000000u;
+// with records: slots of the rays for the coarse part, and of those that left the grid
+struct MarchPoolRec : MarchPool {
+    uint8_t keep[kMarchRays], away[kMarchRays];
+};
+// id: the ray's index in the tile; kMarchSuper set for the SuperSparse marcher.
+// Of a ray that left the grid also twice its next test's distance from bit 8
+// on, and kMarchFine where that test is one of the fine part.
+constexpr uint32_t kMarchSuper = 0x80000000u, kMarchRay = 0xffu, kMarchFine = 1u << 20;
 
 // x + 1.5 * 2^(23 - k), rounded down, holds floor(2^k x) in its low bits
 // (|x| < 2^20): floor(x / 4), floor(x / 2) and floor(2 x) of a position.
@@ -138,14 +148,13 @@ __device__ __forceinline__ bool march_outside(const GridView& g, f3 p, f3 e) {
 constexpr float kMarchEdge = 1.0f / 32.0f;
 // The N tests from p on, s apart: bit j of the result set where test j finds a
 // voxel. q becomes the position after them. `in`: p is known to lie in [0, n)
-// (it becomes so for q's batch); skip: that nothing can be hit; small:
-// march_small(s); left: nothing can be hit from q on. lanes: those that call it
+// (it becomes so for q's batch); small: march_small(s); left: nothing can be hit from q on. lanes: those that call it
 // together, from a vote of the whole warp. EDGE: tests at once on the grid's
 // edge (2 for sparse rays, 30,000 along an axis 41 -> 33 us; the light passes
 // have no room for it, 1080p with records 418 -> 464 us).
 template <bool FINE, int N, int EDGE>
-__device__ __forceinline__ unsigned march_tests(unsigned lanes, const GridView& g, f3 p, f3 s, f3& q, bool& in, bool skip,
-                                                bool small, bool& left) {
+__device__ __forceinline__ unsigned march_tests(unsigned lanes, const GridView& g, f3 p, f3 s, f3& q, bool& in, bool small,
+                                                bool& left) {
     // where the last test lies, to less than what the bounds leave
     const f3 e = mk(__fmaf_rn(s.x, (float)(N - 1), p.x), __fmaf_rn(s.y, (float)(N - 1), p.y),
                     __fmaf_rn(s.z, (float)(N - 1), p.z));
@@ -154,7 +163,7 @@ __device__ __forceinline__ unsigned march_tests(unsigned lanes, const GridView& 
     unsigned hits = 0u;
     q = p;
     const bool inner = in && in_e;  // every position from p to e is inside
-    const bool none = !inner && (skip || (small && march_outside(g, p, e)));
+    const bool none = !inner && small && march_outside(g, p, e);
     // One lane on the grid's edge sends its whole warp through the tests that
     // look at every position: a branch per lane would run both loops.
     if (__all_sync(lanes, inner || none)) {
@@ -188,23 +197,26 @@ __device__ __forceinline__ float march_dcoarse(uint32_t id) { return (id & kMarc
 // last, steps) is called once per ray that ends in this part: t the hit
 // distance or dist, `last` the last position tested, steps the tests made (the
 // last two for REC only). Returns the number of rays that go on to the coarse
-// part, which are the pool's first ones then. Rays that ended wait until no
-// more than kMarchRefill lanes run: their ends and the refill cost about as
-// much as a batch of tests.
-template <bool FINE, bool REC, int EDGE, class Done>
-__device__ __forceinline__ int march_part(const GridView& g, MarchPool& P, int count, Done done) {
+// part: the pool's first ones then, or with REC those of P.keep. With REC rays
+// that left the grid are put by in P.away, `away` of them. Rays that ended wait
+// until no more than kMarchRefill lanes run: their ends and the refill cost
+// about as much as a batch of tests.
+template <bool FINE, bool REC, int EDGE, class Pool, class Done>
+__device__ __forceinline__ int march_part(const GridView& g, Pool& P, int count, int& away, Done done) {
     constexpr int N = kMarchBatch;
-    int base = 0, kept = 0;
-    bool busy = false, in = false, ghost = false, small = true;
+    int base = 0, kept = 0, slot = 0;
+    bool busy = false, in = false, small = true;
     f3 p = mk(0.0f, 0.0f, 0.0f), s = p;
     float d = 0.0f, ds = 0.0f, lim = 0.0f, dist = 0.0f;
     uint32_t id = 0;
     for (;;) {
         const unsigned idle = __ballot_sync(0xffffffffu, !busy);
+        bool off = false;  // left the grid, tests to go
         if (base < count) {
             const int at = base + __popc(idle & march_lanes_below());
             if (!busy && at < count) {
-                const float4 a = P.a[at], b = P.b[at];
+                if constexpr (REC) slot = FINE ? at : P.keep[at];
+                const float4 a = P.a[REC ? slot : at], b = P.b[REC ? slot : at];
                 p = mk(a.x, a.y, a.z);
                 s = mk(b.x, b.y, b.z);
                 dist = a.w;
@@ -213,36 +225,30 @@ __device__ __forceinline__ int march_part(const GridView& g, MarchPool& P, int c
                 d = FINE ? ds * (float)(kMarchFirst + 1) : march_dcoarse(id);
                 lim = FINE ? 16.0f : (dist < 164.0f ? dist : 164.0f);
                 in = p.x >= 0.0f && p.y >= 0.0f && p.z >= 0.0f && march_inside(g, p);
-                ghost = REC && march_gone(g, p, s);
                 small = march_small(s);
-                busy = true;
+                off = REC && FINE && march_gone(g, p, s);
+                busy = !off;
             }
             base = min(base + __popc(idle), count);
             __syncwarp();
         } else if (idle == 0xffffffffu) {
             break;
         }
+        float next = d;  // of the tests to go, and whether they are fine ones
+        bool fine = FINE;
         const int waiting = base < count ? kMarchRefill : 0;
         bool run = busy, left = false;
         unsigned hits = 0u, lanes = __ballot_sync(0xffffffffu, run);
         do {
-            if (REC && run && ghost) {
-                // out of the grid for good: on to the last tests without looking
-                for (int b = 0; b < 8 && d + (float)N * ds < lim; b++) {
-                    for (int j = 0; j < N; j++) p = add(p, s);
-                    d = d + (float)N * ds;
-                }
-            }
             if (run) {
                 f3 q;
-                hits = march_tests<FINE, N, EDGE>(lanes, g, p, s, q, in, REC && ghost, small, left);
+                hits = march_tests<FINE, N, EDGE>(lanes, g, p, s, q, in, small, left);
                 const float dn = d + (float)N * ds;  // small multiples of 0.5: exact
-                if (hits != 0u || !(dn < lim) || (left && !REC)) {
+                if (hits != 0u || !(dn < lim) || left) {
                     run = false;
                 } else {
                     p = q;
                     d = dn;
-                    ghost = REC && (ghost || left);
                 }
             }
             lanes = __ballot_sync(0xffffffffu, run);
@@ -254,28 +260,49 @@ __device__ __forceinline__ int march_part(const GridView& g, MarchPool& P, int c
             for (int j = 1; j < N; j++) nv += d + (float)j * ds < lim ? 1 : 0;
             const int first = __ffs(hits) - 1;
             const bool hit = hits != 0u && first < nv;
-            const float dcoarse = march_dcoarse(id);
-            if (FINE && !hit && !(d + (float)N * ds < lim) && dcoarse < (dist < 164.0f ? dist : 164.0f)) {
+            const float dcoarse = march_dcoarse(id), dn = d + (float)N * ds;
+            if (FINE && !hit && !(dn < lim) && dcoarse < (dist < 164.0f ? dist : 164.0f)) {
                 for (int j = 0; j < nv; j++) p = add(p, s);
-                keep = REC || !march_gone(g, p, s);
+                keep = !march_gone(g, p, s);
+                s = mul(s, 2.0f);
+                off = REC && !keep;
+                next = dcoarse;
+                fine = false;
+            } else if (REC && !hit && dn < lim) {
+                for (int j = 0; j < N; j++) p = add(p, s);
+                off = true;
+                next = dn;
             }
-            if (!keep) {
+            if (!keep && !off) {
                 const int k = hit ? first : nv - 1;
                 const float t = d + (float)k * ds;
                 if (REC)
                     for (int j = 0; j < k; j++) p = add(p, s);
                 const int steps =
                     REC ? (int)((t - (FINE ? ds : dcoarse)) / ds) + 1 + (FINE ? 0 : ((id & kMarchSuper) ? 6 : 31)) : 0;
-                done(id & ~kMarchSuper, hit, hit ? t : dist, FINE, p, steps);
+                done(id & kMarchRay, hit, hit ? t : dist, FINE, p, steps);
             }
             busy = false;
         }
-        if (FINE) {
+        if constexpr (REC) {
+            const unsigned km = __ballot_sync(0xffffffffu, keep), om = __ballot_sync(0xffffffffu, off);
+            if (keep || off) {
+                const uint32_t rest = off ? (uint32_t)(2.0f * next) << 8 | (fine ? kMarchFine : 0u) : 0u;
+                P.a[slot] = make_float4(p.x, p.y, p.z, dist);
+                P.b[slot] = make_float4(s.x, s.y, s.z, __uint_as_float(id | rest));
+                if (keep)
+                    P.keep[kept + __popc(km & march_lanes_below())] = (uint8_t)slot;
+                else
+                    P.away[away + __popc(om & march_lanes_below())] = (uint8_t)slot;
+            }
+            kept += __popc(km);
+            away += __popc(om);
+        } else if constexpr (FINE) {
             const unsigned km = __ballot_sync(0xffffffffu, keep);
             if (keep) {
                 const int at = kept + __popc(km & march_lanes_below());
                 P.a[at] = make_float4(p.x, p.y, p.z, dist);
-                P.b[at] = make_float4(s.x * 2.0f, s.y * 2.0f, s.z * 2.0f, __uint_as_float(id));
+                P.b[at] = make_float4(s.x, s.y, s.z, __uint_as_float(id));
             }
             kept += __popc(km);
         }
@@ -284,13 +311,41 @@ __device__ __forceinline__ int march_part(const GridView& g, MarchPool& P, int c
     return kept;
 }
 
+// The records of rays that left the grid: their last position and test count.
+template <class Done>
+__device__ __forceinline__ void march_away(const MarchPoolRec& P, int count, Done done) {
+    for (int i = threadIdx.x & 31; i < count; i += 32) {
+        const float4 a = P.a[P.away[i]], b = P.b[P.away[i]];
+        f3 p = mk(a.x, a.y, a.z), s = mk(b.x, b.y, b.z), last = p;
+        const uint32_t id = __float_as_uint(b.w);
+        float d = 0.5f * (float)(id >> 8 & 0x1ffu), ds = march_step0(id);
+        if (id & kMarchFine) {
+            for (; d < 16.0f; d += ds) {
+                last = p;
+                p = add(p, s);
+            }
+            s = mul(s, 2.0f);
+        }
+        ds *= 2.0f;
+        const float lim = a.w < 164.0f ? a.w : 164.0f, dcoarse = march_dcoarse(id);
+        for (; d < lim; d += ds) {
+            last = p;
+            p = add(p, s);
+        }
+        const int coarse = (int)((d - dcoarse) / ds);
+        done(id & kMarchRay, false, a.w, coarse == 0, last, ((id & kMarchSuper) ? 6 : 31) + coarse);
+    }
+}
+
 // Both parts. The warp has written the pool's rays; those whose origin or
 // direction is outside ray_domain_ok are left out by the caller (misses).
-template <bool REC, int EDGE = 1, class Done>
-__device__ __forceinline__ void march_pool(const GridView& g, MarchPool& P, int count, Done done) {
+template <bool REC, int EDGE = 1, class Pool, class Done>
+__device__ __forceinline__ void march_pool(const GridView& g, Pool& P, int count, Done done) {
     __syncwarp();
-    const int kept = march_part<true, REC, EDGE>(g, P, count, done);
-    march_part<false, REC, EDGE>(g, P, kept, done);
+    int away = 0;
+    const int kept = march_part<true, REC, EDGE>(g, P, count, away, done);
+    march_part<false, REC, EDGE>(g, P, kept, away, done);
+    if constexpr (REC) march_away(P, away, done);
 }
 
 // The first kMarchFirst tests of one ray per lane with `on` set (a quarter of
@@ -307,16 +362,16 @@ __device__ __forceinline__ void march_push(const GridView& g, MarchPool& P, int&
     const unsigned lanes = __ballot_sync(0xffffffffu, on);
     if (on) {
         bool in = o.x >= 0.0f && o.y >= 0.0f && o.z >= 0.0f && march_inside(g, o), left = false;
-        const unsigned hits = march_tests<true, kMarchFirst, EDGE>(lanes, g, o, s, q, in, false, march_small(s), left);
+        const unsigned hits = march_tests<true, kMarchFirst, EDGE>(lanes, g, o, s, q, in, march_small(s), left);
         if (hits) {
             const int k = __ffs(hits) - 1;
             f3 p = o;
             if (REC)
                 for (int j = 0; j < k; j++) p = add(p, s);
-            done(id & ~kMarchSuper, true, step0 * (float)(k + 1), true, p, k + 1);
+            done(id & kMarchRay, true, step0 * (float)(k + 1), true, p, k + 1);
             on = false;
         } else if (!REC && left) {
-            done(id & ~kMarchSuper, false, dist, true, o, 0);
+            done(id & kMarchRay, false, dist, true, o, 0);
             on = false;
         }
     }

@@ -121,15 +121,15 @@ __global__ void __launch_bounds__(128) k_super_rays(GridView g, const float* __r
 }
 
 // Sparse rays with records: `tile` rays (a multiple of 32) per warp. 1 M rays
-// from random points 145 us (246 one ray a thread). An image's rays, which run
-// alike, gain nothing from a pool: 1 M of one view 200 us, 161 one a thread.
+// from random points 133 us (246 one ray a thread). An image's rays, which run
+// alike, gain nothing from a pool: 1 M of one view 185 us, 161 one a thread.
 __global__ void __launch_bounds__(32 * kMarchWarps, kMarchBlocks) k_march_rays(const __grid_constant__ GridView g,
                                                                     const float* __restrict__ rays, int64_t n, int tile,
                                                                     vxl_ray_record* __restrict__ rec) {
-    __shared__ MarchPool pools[kMarchWarps];
+    __shared__ MarchPoolRec pools[kMarchWarps];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t at = ((int64_t)blockIdx.x * kMarchWarps + warp) * tile;
-    MarchPool& P = pools[warp];
+    MarchPoolRec& P = pools[warp];
     auto done = [&](uint32_t id, bool hit, float t, bool fine, f3 last, int steps) {
         store_record(rec + at + id, march_hit(hit, t, fine, last, steps));
     };
@@ -249,11 +249,12 @@ __global__ void __launch_bounds__(32 * kMarchWarps, kMarchBlocks)
     k_light_ambient(const __grid_constant__ GridView g, const float* __restrict__ wcp_in, const float* __restrict__ nrm,
                     const float* __restrict__ depth, const float4* __restrict__ noise, int64_t npix, f3 sun, int tile,
                     float* __restrict__ shadow, float* __restrict__ irr, vxl_ray_record* __restrict__ rec) {
-    __shared__ MarchPool pools[kMarchWarps];
+    using Pool = std::conditional_t<REC, MarchPoolRec, MarchPool>;
+    __shared__ Pool pools[kMarchWarps];
     __shared__ float res[kMarchWarps][kMarchRays];  // t of ray 2 * pixel + {0: sun, 1: hemisphere}
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t at = ((int64_t)blockIdx.x * kMarchWarps + warp) * tile;
-    MarchPool& P = pools[warp];
+    Pool& P = pools[warp];
     float* rt = res[warp];
     auto done = [&](uint32_t id, bool hit, float t, bool fine, f3 last, int steps) {
         if (hit) rt[id] = t;
@@ -305,11 +306,12 @@ __global__ void __launch_bounds__(32 * kMarchWarps, kMarchBlocks)
                        const float* __restrict__ nrm, const float* __restrict__ view_r,
                        const float* __restrict__ rough, const float4* __restrict__ noise, int64_t npix, int tile,
                        float* __restrict__ t_out, vxl_ray_record* __restrict__ rec) {
-    __shared__ MarchPool pools[kMarchWarps];
+    using Pool = std::conditional_t<REC, MarchPoolRec, MarchPool>;
+    __shared__ Pool pools[kMarchWarps];
     __shared__ float res[kMarchWarps][kMarchRays];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t at = ((int64_t)blockIdx.x * kMarchWarps + warp) * tile;
-    MarchPool& P = pools[warp];
+    Pool& P = pools[warp];
     float* rt = res[warp];
     auto done = [&](uint32_t id, bool hit, float t, bool fine, f3 last, int steps) {
         if (hit) rt[id] = t;
