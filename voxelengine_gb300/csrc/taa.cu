@@ -43,8 +43,16 @@ struct TaaIn {
 };
 
 // The pass's launches follow one another with their starts overlapped (taa_launch):
-// this waits for the one before to end and its writes to be seen.
-__device__ __forceinline__ void after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// this waits for the one before to end and its writes to be seen. The pointers
+// to what the pass itself has written are given anew after the wait: loads
+// through the read-only path, which the compiler may take for constants of the
+// launch, cannot be moved before it then.
+template <class... P>
+__device__ __forceinline__ void after_previous(P&... p) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    auto anew = [](auto& q) { asm volatile("" : "+l"(q)::"memory"); };
+    (anew(p), ...);
+}
 
 __device__ __forceinline__ float gmax(float x, float y) { return (x < y) ? y : x; }
 __device__ __forceinline__ float gmin(float x, float y) { return (y < x) ? y : x; }
@@ -406,7 +414,7 @@ __global__ void __launch_bounds__(THREADS, THREADS == 128 ? 8 : 2) k_taa_edge(co
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const float iResx = 1.0f / (float)I.W, iResy = 1.0f / (float)I.H;
     const unsigned n = (unsigned)I.W * (unsigned)I.H;
-    after_previous();
+    after_previous(rec, motion_max, list);
     const int few = list[0], many = list[1], count = many >= apart ? few : few + many;
     const int group = min(kEdgeGroup, (count + (int)gridDim.x - 1) / (int)gridDim.x);
     for (int k = blockIdx.x * group; k < count; k += gridDim.x * group) {
@@ -460,7 +468,7 @@ constexpr int kManyThreads = 128;
 __global__ void __launch_bounds__(kManyThreads, 4) k_taa_many(const TaaIn I, const float4* __restrict__ rec,
                                                               const int* __restrict__ list, int apart,
                                                               float* __restrict__ out) {
-    after_previous();
+    after_previous(rec, list);
     const int many = list[1], lane = threadIdx.x & 31;
     if (many >= apart) {
         const unsigned n = (unsigned)I.W * (unsigned)I.H;
@@ -537,7 +545,7 @@ __global__ void __launch_bounds__(32 * kTaaRows, BLOCKS) k_taa(const TaaIn I, co
     const int i = valid ? py * W + px : 0;
     const size_t n = (size_t)W * H;
     const float4* mat = reinterpret_cast<const float4*>(I.material);
-    after_previous();
+    after_previous(rec, motion_max, list);
     const bool still = taa_still(W, H, (int)(blockIdx.x * WIDE / kPackW), (int)(blockIdx.y * kTaaRows / kPackH), motion_max);
     const float GR = 2.118033988749895f;
     const float iResx = 1.0f / (float)W, iResy = 1.0f / (float)H;
